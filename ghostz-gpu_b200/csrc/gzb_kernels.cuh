@@ -1205,29 +1205,13 @@ __device__ __forceinline__ int lane_row(const GappedJob &job, const int *sm, Lan
   return kLaneRunning;
 }
 
-template <int W>
-__device__ inline GappedOut gapped_extend_lane(const GappedJob &job, const int *sm,
-                                               LaneBand<W> band, uint32_t qpos, uint32_t dpos,
-                                               bool reverse) {
-  LaneExt x;
-  int st = lane_init(job, band, x, job.query + qpos, job.db + dpos, reverse);
-  while (st == kLaneRunning) st = lane_row(job, sm, band, x);
-  GappedOut out;
-  out.overflow = st == kLaneOverflow || x.ovf;
-  out.score = x.maxs;
-  out.pos0 = x.mp0;
-  out.pos1 = x.mp1;
-  out.cells = x.cells;
-  return out;
-}
-
 }  // namespace gzb
 
 namespace gzb {
 
 // ---------------------------------------------------------------------------
 // Gapped extension, one thread per extension, flattened.  Same recurrence as
-// gapped_extend_lane, but the row loop, the cell loop and the loop over
+// lane_init / lane_row, but the row loop, the cell loop and the loop over
 // extensions are one loop that advances every lane by one DP cell per
 // iteration: a lane that reaches the end of its row, or of its extension,
 // does that bookkeeping and carries on with its next cell, so the lanes of a

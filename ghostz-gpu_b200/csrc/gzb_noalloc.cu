@@ -41,13 +41,12 @@
 namespace gzb {
 
 // kernels of the regular gapped extender (gzb_operators.cu)
-__global__ void gapped_lane_kernel(GappedJob job, const int32_t *__restrict__ matrix,
-                                   int number_letters, int stride, size_t n,
-                                   const uint32_t *__restrict__ order, int reverse,
-                                   const uint8_t *__restrict__ dir, uint32_t *qpos,
-                                   uint32_t *dpos, int32_t *scores, uint32_t *spill,
-                                   uint32_t *spill_count, unsigned long long *cells_total,
-                                   uint32_t *cells_out, const uint64_t *n_dev);
+int launch_gapped_static(unsigned blocks, const GappedJob &job, const int32_t *matrix,
+                         int number_letters, int stride, size_t n, const uint32_t *order,
+                         int reverse, const uint8_t *dir, uint32_t *qpos, uint32_t *dpos,
+                         int32_t *scores, uint32_t *spill, uint32_t *spill_count,
+                         unsigned long long *cells_total, uint32_t *cells_out, cudaStream_t s,
+                         const uint64_t *n_dev);
 __global__ void gapped_warp_kernel(GappedJob job, const int32_t *__restrict__ matrix,
                                    int number_letters, int stride, const uint32_t *list,
                                    const uint32_t *list_count, int reverse,
@@ -142,11 +141,10 @@ extern "C" int gzb_gapped_extend_one_side_score_only_noalloc(
   GZB_CUDA(cudaGetDevice(&dev));
   GZB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const size_t blocks = (size + 127) / 128, cap = (size_t)sms * 40;
-  gapped_lane_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 128, 0, s>>>(
-      job, d_score_matrix, (int)number_letters, stride, size, nullptr, reverse, nullptr,
-      d_query_concatenated_positions, d_database_positions, d_scores, spill1, counters, cells,
-      nullptr, nullptr);
-  GZB_CUDA(cudaGetLastError());
+  GZB_TRY(launch_gapped_static((unsigned)(blocks < cap ? blocks : cap), job, d_score_matrix,
+                               (int)number_letters, stride, size, nullptr, reverse, nullptr,
+                               d_query_concatenated_positions, d_database_positions, d_scores,
+                               spill1, counters, cells, nullptr, s, nullptr));
   const uint32_t *serial_list = spill1, *serial_count = counters;
   if (warp_path_exact(cutoff)) {
     gapped_warp_kernel<<<sms * 4, 256, 0, s>>>(job, d_score_matrix, (int)number_letters,

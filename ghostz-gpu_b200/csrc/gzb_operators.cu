@@ -12,6 +12,7 @@
 #include "ghostz_b200.h"
 #include "gzb_common.h"
 #include "gzb_kernels.cuh"
+#include "gzb_row.cuh"
 
 namespace gzb {
 
@@ -203,33 +204,106 @@ __device__ __forceinline__ void store_result(uint32_t e, uint32_t q, uint32_t d,
   scores[e] = o.score;
 }
 
+// One extension on one thread, a database row at a time.  FAST: the grouped
+// rows of gzb_row.cuh, for the parameters row_dp_exact admits (three quarters
+// of the other form's time, see there); else lane_init / lane_row, for every
+// X-drop.
+__host__ __device__ constexpr int lane_table_words(bool fast) {
+  return fast ? kRowTableWords : kMatrixStride * kMatrixStride;
+}
+
+template <int W, bool FAST>
+struct LaneWork;
+
+template <int W>
+struct LaneWork<W, false> {
+  const int *tbl;
+  LaneBand<W> band;
+  LaneExt x;
+  __device__ __forceinline__ LaneWork(const GappedJob &job, int *tbl_, uint32_t *cells,
+                                      uint8_t *res, const int32_t *matrix, int number_letters,
+                                      int stride)
+      : tbl(tbl_), band(cells, res, kLaneBlock, (int)threadIdx.x) {
+    load_matrix(tbl_, matrix, number_letters, stride);
+    __syncthreads();
+  }
+  __device__ __forceinline__ int init(const GappedJob &job, uint32_t q, uint32_t d, bool rev) {
+    return lane_init(job, band, x, job.query + q, job.db + d, rev);
+  }
+  // the next row, if st is kLaneRunning
+  __device__ __forceinline__ int step(const GappedJob &job, int st) {
+    return st == kLaneRunning ? lane_row(job, tbl, band, x) : st;
+  }
+  __device__ __forceinline__ bool overflow(int st) const { return st == kLaneOverflow || x.ovf; }
+  __device__ __forceinline__ int score() const { return x.maxs; }
+  __device__ __forceinline__ int pos0() const { return x.mp0; }
+  __device__ __forceinline__ int pos1() const { return x.mp1; }
+};
+
+template <int W>
+struct LaneWork<W, true> {
+  uint32_t tbl;  // shared-memory address
+  RowBand<W, kLaneBlock> band;
+  RowExt x;
+  bool fits;  // the matrix (a larger one hands every extension on)
+  __device__ __forceinline__ LaneWork(const GappedJob &job, int *tbl_, uint32_t *cells,
+                                      uint8_t *res, const int32_t *matrix, int number_letters,
+                                      int stride)
+      : tbl((uint32_t)__cvta_generic_to_shared(tbl_)) {
+    band.cell = (uint32_t)__cvta_generic_to_shared(cells) + 16 * threadIdx.x;
+    band.res = (uint32_t)__cvta_generic_to_shared(res) + 4 * threadIdx.x;
+    fits = load_row_table(tbl_, job, matrix, number_letters, stride);
+  }
+  __device__ __forceinline__ int init(const GappedJob &job, uint32_t q, uint32_t d, bool rev) {
+    const int st = row_init<W, kLaneBlock>(job, band, x, job.query + q, job.db + d, rev);
+    return fits ? st : kLaneOverflow;
+  }
+  __device__ __forceinline__ int step(const GappedJob &job, int st) {
+    return row_step<W, kLaneBlock>(job, tbl, band, x, st);
+  }
+  __device__ __forceinline__ bool overflow(int st) const { return st == kLaneOverflow; }
+  __device__ __forceinline__ int score() const { return x.best; }
+  __device__ __forceinline__ int pos0() const { return x.pos0(); }
+  __device__ __forceinline__ int pos1() const { return x.pos1(); }
+};
+
+template <bool FAST>
 __global__ void __launch_bounds__(kLaneBlock)
 gapped_lane_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number_letters,
                    int stride, size_t n, const uint32_t *__restrict__ order, int reverse,
                    const uint8_t *__restrict__ dir, uint32_t *qpos, uint32_t *dpos,
                    int32_t *scores, uint32_t *spill, uint32_t *spill_count,
                    unsigned long long *cells_total, uint32_t *cells_out, const uint64_t *n_dev) {
-  __shared__ int sm[kMatrixStride * kMatrixStride];
-  __shared__ uint32_t cells_s[kLaneW * kLaneBlock];
-  __shared__ uint8_t res_s[kLaneW * kLaneBlock];
+  __shared__ int sm[lane_table_words(FAST)];
+  __shared__ __align__(16) uint32_t cells_s[kLaneW * kLaneBlock];
+  __shared__ __align__(4) uint8_t res_s[kLaneW * kLaneBlock];
   if (n_dev) n = *n_dev;
-  load_matrix(sm, matrix, number_letters, stride);
-  __syncthreads();
-  LaneBand<kLaneW> band(cells_s, res_s, kLaneBlock, (int)threadIdx.x);
+  LaneWork<kLaneW, FAST> x(job, sm, cells_s, res_s, matrix, number_letters, stride);
   unsigned long long cells = 0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t e = order ? order[i] : (uint32_t)i;
-    const bool rev = dir ? dir[e] != 0 : reverse != 0;
-    const uint32_t q = qpos[e], d = dpos[e];
-    GappedOut o = gapped_extend_lane(job, sm, band, q, d, rev);
-    if (o.overflow) {
+  const size_t lane = threadIdx.x & 31;
+  for (size_t i0 = blockIdx.x * (size_t)blockDim.x + (threadIdx.x & ~31u); i0 < n;
+       i0 += (size_t)gridDim.x * blockDim.x) {
+    const size_t i = i0 + lane;
+    uint32_t e = 0, q = 0, d = 0;
+    int st = kLaneDone;
+    if (i < n) {
+      e = order ? order[i] : (uint32_t)i;
+      const bool rev = dir ? dir[e] != 0 : reverse != 0;
+      q = qpos[e];
+      d = dpos[e];
+      st = x.init(job, q, d, rev);
+    }
+    while (__any_sync(0xffffffffu, st == kLaneRunning)) st = x.step(job, st);
+    if (i >= n) {
+    } else if (x.overflow(st)) {
       spill[atomicAdd(spill_count, 1u)] = e;
       if (cells_out) cells_out[e] = 0xFFFFFFFFu;
     } else {
-      cells += o.cells;
-      store_result(e, q, d, o, qpos, dpos, scores);
-      if (cells_out) cells_out[e] = (uint32_t)o.cells;
+      cells += x.x.cells;
+      qpos[e] = q + (uint32_t)x.pos0();
+      dpos[e] = d + (uint32_t)x.pos1();
+      scores[e] = x.score();
+      if (cells_out) cells_out[e] = x.x.cells;
     }
   }
   cells += __shfl_down_sync(0xffffffffu, cells, 16);
@@ -267,6 +341,7 @@ gapped_flat_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
 // of similar cost placed next to each other keep the warp's lanes busy.
 // cells_out (optional) records every extension's DP cells, UINT32_MAX when
 // it was handed to the fallback.
+template <bool FAST>
 __global__ void __launch_bounds__(kLaneBlock)
 gapped_lane_queue_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number_letters,
                          int stride, uint64_t n, const uint32_t *__restrict__ order,
@@ -274,13 +349,11 @@ gapped_lane_queue_kernel(GappedJob job, const int32_t *__restrict__ matrix, int 
                          uint32_t *qpos, uint32_t *dpos, int32_t *scores, uint32_t *spill,
                          uint32_t *spill_count, unsigned long long *cells_total,
                          uint32_t *cells_out, const uint64_t *n_dev) {
-  __shared__ int sm[kMatrixStride * kMatrixStride];
-  __shared__ uint32_t cells_s[kLaneW * kLaneBlock];
-  __shared__ uint8_t res_s[kLaneW * kLaneBlock];
+  __shared__ int sm[lane_table_words(FAST)];
+  __shared__ __align__(16) uint32_t cells_s[kLaneW * kLaneBlock];
+  __shared__ __align__(4) uint8_t res_s[kLaneW * kLaneBlock];
   if (n_dev) n = *n_dev;
-  load_matrix(sm, matrix, number_letters, stride);
-  __syncthreads();
-  LaneBand<kLaneW> band(cells_s, res_s, kLaneBlock, (int)threadIdx.x);
+  LaneWork<kLaneW, FAST> x(job, sm, cells_s, res_s, matrix, number_letters, stride);
   const int lane = threadIdx.x & 31;
   unsigned long long cells = 0;
   for (;;) {
@@ -289,18 +362,26 @@ gapped_lane_queue_kernel(GappedJob job, const int32_t *__restrict__ matrix, int 
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= n) break;
     const uint64_t i = base + lane;
+    uint32_t e = 0, q = 0, d = 0;
+    int st = kLaneDone;
     if (i < n) {
-      const uint32_t e = order ? order[i] : (uint32_t)i;
+      e = order ? order[i] : (uint32_t)i;
       const bool rev = dir ? dir[e] != 0 : reverse != 0;
-      const uint32_t q = qpos[e], d = dpos[e];
-      GappedOut o = gapped_extend_lane(job, sm, band, q, d, rev);
-      if (o.overflow) {
+      q = qpos[e];
+      d = dpos[e];
+      st = x.init(job, q, d, rev);
+    }
+    while (__any_sync(0xffffffffu, st == kLaneRunning)) st = x.step(job, st);
+    if (i < n) {
+      if (x.overflow(st)) {
         spill[atomicAdd(spill_count, 1u)] = e;
         if (cells_out) cells_out[e] = 0xFFFFFFFFu;
       } else {
-        cells += o.cells;
-        store_result(e, q, d, o, qpos, dpos, scores);
-        if (cells_out) cells_out[e] = o.cells > 0xFFFFFFFEull ? 0xFFFFFFFEu : (uint32_t)o.cells;
+        cells += x.x.cells;
+        qpos[e] = q + (uint32_t)x.pos0();
+        dpos[e] = d + (uint32_t)x.pos1();
+        scores[e] = x.score();
+        if (cells_out) cells_out[e] = x.x.cells;
       }
     }
     __syncwarp();
@@ -331,7 +412,7 @@ constexpr size_t rows_band_bytes(int W) {
   return rows_band_static(W) ? 0 : (size_t)W * kLaneBlock * 5;
 }
 
-template <int W>
+template <int W, bool FAST>
 __global__ void __launch_bounds__(kLaneBlock)
 gapped_rows_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number_letters,
                    int stride, uint64_t n, const uint32_t *__restrict__ order,
@@ -339,40 +420,36 @@ gapped_rows_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
                    uint32_t *qpos, uint32_t *dpos, int32_t *scores, uint32_t *spill,
                    uint32_t *spill_count, unsigned long long *cells_total,
                    uint32_t *cells_out, int refill_threshold, const uint64_t *n_dev) {
-  __shared__ int sm[kMatrixStride * kMatrixStride];
+  __shared__ int sm[lane_table_words(FAST)];
   constexpr bool kStatic = rows_band_static(W);
-  __shared__ uint32_t cells_st[kStatic ? W * kLaneBlock : 1];
-  __shared__ uint8_t res_st[kStatic ? W * kLaneBlock : 1];
+  __shared__ __align__(16) uint32_t cells_st[kStatic ? W * kLaneBlock : 1];
+  __shared__ __align__(4) uint8_t res_st[kStatic ? W * kLaneBlock : 1];
   extern __shared__ __align__(16) uint8_t rows_band[];
   // [W][kLaneBlock] each
   uint32_t *cells_s = kStatic ? cells_st : reinterpret_cast<uint32_t *>(rows_band);
   uint8_t *res_s = kStatic ? res_st : rows_band + (size_t)W * kLaneBlock * 4;
   if (n_dev) n = *n_dev;
-  load_matrix(sm, matrix, number_letters, stride);
-  __syncthreads();
-  LaneBand<W> band(cells_s, res_s, kLaneBlock, (int)threadIdx.x);
-  LaneExt x;
+  LaneWork<W, FAST> x(job, sm, cells_s, res_s, matrix, number_letters, stride);
   uint32_t e = 0, q = 0, d = 0;
   bool have = false, done = false;
   unsigned long long cells = 0;
   for (;;) {
-    int st = kLaneRunning;
-    if (have) st = lane_row(job, sm, band, x);
+    int st = x.step(job, have ? kLaneRunning : kLaneDone);
     const unsigned idle = __ballot_sync(0xffffffffu, !done && (!have || st != kLaneRunning));
     const unsigned busy = __ballot_sync(0xffffffffu, have && st == kLaneRunning);
     if (idle == 0 && busy == 0) break;
     const bool refill = __popc(idle) >= refill_threshold || busy == 0;
     while (have ? st != kLaneRunning : (refill && !done)) {
       if (have) {  // the extension ended: write it out
-        if (st == kLaneOverflow || x.ovf) {
+        if (x.overflow(st)) {
           spill[atomicAdd(spill_count, 1u)] = e;
           if (cells_out) cells_out[e] = 0xFFFFFFFFu;
         } else {
-          cells += x.cells;
-          qpos[e] = q + (uint32_t)x.mp0;
-          dpos[e] = d + (uint32_t)x.mp1;
-          scores[e] = x.maxs;
-          if (cells_out) cells_out[e] = x.cells;
+          cells += x.x.cells;
+          qpos[e] = q + (uint32_t)x.pos0();
+          dpos[e] = d + (uint32_t)x.pos1();
+          scores[e] = x.score();
+          if (cells_out) cells_out[e] = x.x.cells;
         }
         have = false;
         st = kLaneRunning;
@@ -385,7 +462,7 @@ gapped_rows_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
       const bool rev = dir ? dir[e] != 0 : reverse != 0;
       q = qpos[e];
       d = dpos[e];
-      st = lane_init(job, band, x, job.query + q, job.db + d, rev);
+      st = x.init(job, q, d, rev);
       have = true;
     }
   }
@@ -401,19 +478,18 @@ gapped_rows_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
 // runs extensions order[t], order[t + T], order[t + 2T], ... (T threads),
 // one database row per step like gapped_rows_kernel, and loads the
 // positions of its next extension while the current one runs.
+template <bool FAST>
 __global__ void __launch_bounds__(kLaneBlock)
 gapped_deal_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number_letters,
                    int stride, uint64_t n, const uint32_t *__restrict__ order, int reverse,
                    const uint8_t *__restrict__ dir, uint32_t *qpos, uint32_t *dpos,
                    int32_t *scores, uint32_t *spill, uint32_t *spill_count,
                    unsigned long long *cells_total, uint32_t *cells_out, const uint64_t *n_dev) {
-  __shared__ int sm[kMatrixStride * kMatrixStride];
-  __shared__ uint32_t cells_s[kLaneW * kLaneBlock];
-  __shared__ uint8_t res_s[kLaneW * kLaneBlock];
+  __shared__ int sm[lane_table_words(FAST)];
+  __shared__ __align__(16) uint32_t cells_s[kLaneW * kLaneBlock];
+  __shared__ __align__(4) uint8_t res_s[kLaneW * kLaneBlock];
   if (n_dev) n = *n_dev;
-  load_matrix(sm, matrix, number_letters, stride);
-  __syncthreads();
-  LaneBand<kLaneW> band(cells_s, res_s, kLaneBlock, (int)threadIdx.x);
+  LaneWork<kLaneW, FAST> x(job, sm, cells_s, res_s, matrix, number_letters, stride);
   const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
   uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   // the next extension of this lane, loaded one extension ahead
@@ -428,24 +504,23 @@ gapped_deal_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
     }
   };
   load_next(i);
-  LaneExt x;
   uint32_t e = 0, q = 0, d = 0;
   bool have = false;
   unsigned long long cells = 0;
   for (;;) {
-    int st = kLaneRunning;
-    if (have) st = lane_row(job, sm, band, x);
+    int st = x.step(job, have ? kLaneRunning : kLaneDone);
+    if (!have) st = kLaneRunning;
     while (st != kLaneRunning || (!have && i < n)) {
       if (have) {  // the extension ended: write it out
-        if (st == kLaneOverflow || x.ovf) {
+        if (x.overflow(st)) {
           spill[atomicAdd(spill_count, 1u)] = e;
           if (cells_out) cells_out[e] = 0xFFFFFFFFu;
         } else {
-          cells += x.cells;
-          qpos[e] = q + (uint32_t)x.mp0;
-          dpos[e] = d + (uint32_t)x.mp1;
-          scores[e] = x.maxs;
-          if (cells_out) cells_out[e] = x.cells;
+          cells += x.x.cells;
+          qpos[e] = q + (uint32_t)x.pos0();
+          dpos[e] = d + (uint32_t)x.pos1();
+          scores[e] = x.score();
+          if (cells_out) cells_out[e] = x.x.cells;
         }
         have = false;
         i += T;
@@ -456,7 +531,7 @@ gapped_deal_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
       d = nd;
       const bool rev = nrev;
       load_next(i + T);
-      st = lane_init(job, band, x, job.query + q, job.db + d, rev);
+      st = x.init(job, q, d, rev);
       have = true;
     }
     if (!__any_sync(0xffffffffu, have)) break;
@@ -553,22 +628,46 @@ static int launch_gapped_group(const GappedJob &job, const int32_t *matrix, int 
   return GZB_OK;
 }
 
-template <int W>
-static int launch_gapped_rows(const GappedTile &tile, const GappedJob &job, const int32_t *matrix,
-                              int number_letters, int stride, uint64_t n, const uint32_t *order,
-                              unsigned long long *queue, int reverse, const uint8_t *dir,
-                              uint32_t *qpos, uint32_t *dpos, int32_t *scores, uint32_t *spill,
-                              uint32_t *spill_count, unsigned long long *cells_total,
-                              uint32_t *cells_out, cudaStream_t s, const uint64_t *n_dev) {
+template <int W, bool FAST>
+static int launch_gapped_rows_as(const GappedTile &tile, const GappedJob &job,
+                                 const int32_t *matrix, int number_letters, int stride,
+                                 uint64_t n, const uint32_t *order, unsigned long long *queue,
+                                 int reverse, const uint8_t *dir, uint32_t *qpos, uint32_t *dpos,
+                                 int32_t *scores, uint32_t *spill, uint32_t *spill_count,
+                                 unsigned long long *cells_total, uint32_t *cells_out,
+                                 cudaStream_t s, const uint64_t *n_dev) {
   const size_t smem = rows_band_bytes(W);
   if (smem)
-    GZB_CUDA(cudaFuncSetAttribute(gapped_rows_kernel<W>,
+    GZB_CUDA(cudaFuncSetAttribute(gapped_rows_kernel<W, FAST>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   uint64_t blocks = 1;
-  GZB_TRY(persistent_blocks(gapped_rows_kernel<W>, kLaneBlock, smem, n, &blocks));
-  gapped_rows_kernel<W><<<(unsigned)blocks, kLaneBlock, smem, s>>>(
+  GZB_TRY(persistent_blocks(gapped_rows_kernel<W, FAST>, kLaneBlock, smem, n, &blocks));
+  gapped_rows_kernel<W, FAST><<<(unsigned)blocks, kLaneBlock, smem, s>>>(
       job, matrix, number_letters, stride, n, order, queue, reverse, dir, qpos, dpos, scores,
       spill, spill_count, cells_total, cells_out, tile.book_threshold, n_dev);
+  return GZB_OK;
+}
+
+template <int W, typename... Args>
+static int launch_gapped_rows(const GappedTile &tile, const GappedJob &job, Args... args) {
+  return row_dp_exact(job.gap_open, job.gap_ext, job.cutoff)
+             ? launch_gapped_rows_as<W, true>(tile, job, args...)
+             : launch_gapped_rows_as<W, false>(tile, job, args...);
+}
+
+// One launch, extensions dealt to threads round-robin, no work queue.
+int launch_gapped_static(unsigned blocks, const GappedJob &job, const int32_t *matrix,
+                         int number_letters, int stride, size_t n, const uint32_t *order,
+                         int reverse, const uint8_t *dir, uint32_t *qpos, uint32_t *dpos,
+                         int32_t *scores, uint32_t *spill, uint32_t *spill_count,
+                         unsigned long long *cells_total, uint32_t *cells_out, cudaStream_t s,
+                         const uint64_t *n_dev) {
+  auto kernel = row_dp_exact(job.gap_open, job.gap_ext, job.cutoff) ? gapped_lane_kernel<true>
+                                                                    : gapped_lane_kernel<false>;
+  kernel<<<blocks, kLaneBlock, 0, s>>>(job, matrix, number_letters, stride, n, order, reverse,
+                                       dir, qpos, dpos, scores, spill, spill_count, cells_total,
+                                       cells_out, n_dev);
+  GZB_CUDA(cudaGetLastError());
   return GZB_OK;
 }
 
@@ -582,6 +681,7 @@ int launch_gapped_thread(const GappedTile &tile, const GappedJob &job, const int
   // (grids sized for n)
   GZB_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s));
   uint64_t blocks = 1;
+  const bool fast = row_dp_exact(job.gap_open, job.gap_ext, job.cutoff);
   const bool group = tile.kernel >= GZB_GAPPED_KERNEL_GROUP4 &&
                      tile.kernel <= GZB_GAPPED_KERNEL_GROUP32 && warp_path_exact(job.cutoff);
   if (group) {
@@ -603,17 +703,17 @@ int launch_gapped_thread(const GappedTile &tile, const GappedJob &job, const int
                                       reverse, dir, qpos, dpos, scores, spill, spill_count,
                                       cells_total, cells_out, s, n_dev));
   } else if (tile.kernel == GZB_GAPPED_KERNEL_DEAL) {
-    GZB_TRY(persistent_blocks(gapped_deal_kernel, kLaneBlock, 0, n, &blocks));
-    gapped_deal_kernel<<<(unsigned)blocks, kLaneBlock, 0, s>>>(
+    auto kernel = fast ? gapped_deal_kernel<true> : gapped_deal_kernel<false>;
+    GZB_TRY(persistent_blocks(kernel, kLaneBlock, 0, n, &blocks));
+    kernel<<<(unsigned)blocks, kLaneBlock, 0, s>>>(
         job, matrix, number_letters, stride, n, order, reverse, dir, qpos, dpos, scores, spill,
         spill_count, cells_total, cells_out, n_dev);
   } else if (tile.kernel == GZB_GAPPED_KERNEL_STATIC) {
-    // one launch, extensions dealt to threads round-robin, no work queue
     blocks = (n + kLaneBlock - 1) / kLaneBlock;
     if (blocks > 148 * 40) blocks = 148 * 40;
-    gapped_lane_kernel<<<(unsigned)blocks, kLaneBlock, 0, s>>>(
-        job, matrix, number_letters, stride, n, order, reverse, dir, qpos, dpos, scores, spill,
-        spill_count, cells_total, cells_out, n_dev);
+    GZB_TRY(launch_gapped_static((unsigned)blocks, job, matrix, number_letters, stride, n, order,
+                                 reverse, dir, qpos, dpos, scores, spill, spill_count,
+                                 cells_total, cells_out, s, n_dev));
   } else if (tile.kernel == GZB_GAPPED_KERNEL_ROWS || tile.kernel >= GZB_GAPPED_KERNEL_GROUP4) {
     // (a group kernel's X-drop outside the warp DP's exact range runs here)
     if (tile.band_width == 32)
@@ -629,8 +729,9 @@ int launch_gapped_thread(const GappedTile &tile, const GappedJob &job, const int
                                      reverse, dir, qpos, dpos, scores, spill, spill_count,
                                      cells_total, cells_out, s, n_dev));
   } else if (tile.kernel == GZB_GAPPED_KERNEL_LANE) {
-    GZB_TRY(persistent_blocks(gapped_lane_queue_kernel, kLaneBlock, 0, n, &blocks));
-    gapped_lane_queue_kernel<<<(unsigned)blocks, kLaneBlock, 0, s>>>(
+    auto kernel = fast ? gapped_lane_queue_kernel<true> : gapped_lane_queue_kernel<false>;
+    GZB_TRY(persistent_blocks(kernel, kLaneBlock, 0, n, &blocks));
+    kernel<<<(unsigned)blocks, kLaneBlock, 0, s>>>(
         job, matrix, number_letters, stride, n, order, queue, reverse, dir, qpos, dpos, scores,
         spill, spill_count, cells_total, cells_out, n_dev);
   } else if (tile.kernel == GZB_GAPPED_KERNEL_FLAT) {
