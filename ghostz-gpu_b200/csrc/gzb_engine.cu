@@ -30,6 +30,7 @@
 #include "gzb_common.h"
 #include "gzb_index.cuh"
 #include "gzb_kernels.cuh"
+#include "gzb_walk.cuh"
 #include "gzb_cost.cuh"
 #include "gzb_traceback.cuh"
 
@@ -433,108 +434,267 @@ struct SeedArgs {
   const uint64_t *units_dev = nullptr;  // unit count on the device (else L.n_units)
 };
 
+__device__ __forceinline__ uint64_t hit_key(const SeedArgs &a, uint32_t qid, uint32_t d,
+                                            uint32_t qp) {
+  return ((uint64_t)qid << (a.dbits + a.qbits)) | ((uint64_t)d << a.qbits) | (uint64_t)qp;
+}
+
 __device__ __forceinline__ void emit_hit(const SeedArgs &a, uint32_t qid, uint32_t d,
                                          uint32_t qp) {
-  const uint64_t key = ((uint64_t)qid << (a.dbits + a.qbits)) |
-                       ((uint64_t)d << a.qbits) | (uint64_t)qp;
-  append(a.hits, a.hit_count, a.hit_cap, key);
+  append(a.hits, a.hit_count, a.hit_cap, hit_key(a, qid, d, qp));
 }
 
 constexpr int kSeedBlock = 256;
 constexpr int kUnitsPerWarp = 256;
 
+// Items waiting in shared memory until 32 of them are there, one stack per
+// warp: a warp finds seeds, member work and hits with whatever lanes have
+// one, and walks or writes them 32 at a time.
+template <typename T>
+struct WarpStack {
+  static constexpr uint32_t kCapacity = 64;  // 31 waiting and 32 more
+  T *item;
+  uint32_t n = 0;  // the same on every lane
+  // the lanes with `have` add theirs (all lanes call it)
+  __device__ __forceinline__ void push(bool have, T v) {
+    const unsigned m = __ballot_sync(0xffffffffu, have);
+    if (have) item[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = v;
+    n += __popc(m);
+    __syncwarp();
+  }
+  // the newest 32 (fewer: all), one per lane; false on lanes without one
+  __device__ __forceinline__ bool pop(T *v) {
+    const uint32_t take = n < 32 ? n : 32, lane = threadIdx.x & 31;
+    n -= take;
+    if (lane < take) *v = item[n + lane];
+    __syncwarp();
+    return lane < take;
+  }
+  // pops into a global list: one atomic for the warp
+  __device__ __forceinline__ void flush(T *list, unsigned long long *count,
+                                        unsigned long long cap) {
+    const uint32_t take = n < 32 ? n : 32, lane = threadIdx.x & 31;
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(count, (unsigned long long)take);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    T v;
+    if (pop(&v) && base + lane < cap) list[base + lane] = v;
+  }
+};
+
+// Shared memory of a seed-search block: the window and walk tables and the
+// warps' stacks.
+struct SeedShared {
+  uint32_t window[kWindowTableBytes / 4];
+  int32_t walk[kWalkTableBytes / 4];
+  uint4 found[kSeedBlock / 32][WarpStack<uint4>::kCapacity];
+  uint2 open[kSeedBlock / 32][WarpStack<uint2>::kCapacity];
+  uint2 member[kSeedBlock / 32][WarpStack<uint2>::kCapacity];
+  uint64_t hit[kSeedBlock / 32][WarpStack<uint64_t>::kCapacity];
+};
+
+// The walks of the seeds a warp finds.  Each seed's window is evaluated
+// first (gzb_walk.cuh: no branches, every lane the same length); the one in
+// ten that this leaves open is walked pair by pair, again 32 together.
+//
+// One walk after another per lane instead (each warp waiting for its longest
+// walk, lanes idle where the distance filter had refused) ran 14.6 of 32
+// lanes an instruction, this 27.  Seed and member kernels together, 1.04 G
+// seeds of 10,000 queries x 1,500,000 proteins: 58.2 -> 47.8 ms; 82 M seeds
+// of 2,000 x 400,000: 5.1 -> 4.3 ms.  What is left (2,000 x 400,000): ALU
+// pipe 63 %, L1 wavefronts 62 %, issue 57 %, 3.4 cycles an instruction
+// waiting for global loads; of the 47.8 ms the search for seeds takes 10,
+// the windows' loads 20, their evaluation 10, the open walks 9.  Three
+// blocks an SM: four (64 registers) 50.6 ms; the windows of the next seeds
+// fetched ahead into registers 55 ms (two blocks); prefetched into L2 54.6.
+struct SeedWalker {
+  const SeedArgs &a;
+  uint32_t window;   // table addresses
+  const char *walk;
+  bool fits;         // the matrix (window tables hold entries up to 127)
+  WarpStack<uint4> found;     // (database position, entry, its position, cutoff and trigger)
+  WarpStack<uint2> open;      // (database position, entry)
+  WarpStack<uint64_t> hit;    // packed hit keys
+  // a thread's counts stay far below 2^32 (that many walk steps would take
+  // one thread seconds)
+  uint32_t n_seed = 0, n_steps = 0;
+
+  __device__ __forceinline__ SeedWalker(const SeedArgs &args, SeedShared &sh) : a(args) {
+    load_walk_table(sh.walk, a.matrix32, a.p.delimiter);
+    window = (uint32_t)__cvta_generic_to_shared(sh.window);
+    walk = reinterpret_cast<const char *>(sh.walk);
+    fits = load_window_table(window, a.matrix32, a.p.delimiter);
+    found.item = sh.found[threadIdx.x >> 5];
+    open.item = sh.open[threadIdx.x >> 5];
+    hit.item = sh.hit[threadIdx.x >> 5];
+  }
+
+  // a seed of every lane with `have`; all lanes call it
+  __device__ __forceinline__ void add(bool have, uint32_t d, uint32_t entry, uint32_t cpos,
+                                      uint32_t ct) {
+    found.push(have, make_uint4(d, entry, cpos, ct));
+    if (found.n >= 32) run_found();
+  }
+
+  __device__ __forceinline__ void finish() {
+    if (found.n) run_found();
+    while (open.n) run_open();
+    while (hit.n) hit.flush(a.hits, a.hit_count, a.hit_cap);
+  }
+
+  __device__ __forceinline__ void run_found() {
+    uint4 v = make_uint4(0, 0, 0, 0);
+    const bool have = found.pop(&v);
+    bool settled = false;
+    if (have) {
+      ++n_seed;
+      const int cutoff = (int)(v.w >> 16), trigger = (int)(int16_t)(v.w & 0xffffu);
+      if (fits && cutoff <= kWalkMaxCutoff) {
+        const uint8_t *qs = a.q + v.z, *ds = a.db + v.x;
+        uint32_t q[16], d[16];
+        WindowWords qw, dw;
+        fetch_window(qs, qw);
+        fetch_window(ds, dw);
+        align_window(qs, qw, q);
+        align_window(ds, dw, d);
+        int steps;
+        settled = walk_window(window, q, d, cutoff, trigger, &steps);
+        if (settled) n_steps += (uint32_t)steps;
+      }
+    }
+    open.push(have && !settled, make_uint2(v.x, v.y));
+    if (open.n >= 32) run_open();
+  }
+
+  __device__ __forceinline__ void run_open() {
+    uint2 v = make_uint2(0, 0);
+    bool is_hit = false;
+    uint64_t key = 0;
+    if (open.pop(&v)) {
+      const uint32_t ct = a.L.entry_ct[v.y], cpos = a.L.entry_cpos[v.y];
+      int steps = 0;
+      is_hit = walk_hit(a.q + cpos, a.db + v.x, walk, (int)(ct >> 16),
+                        (int)(int16_t)(ct & 0xffffu), &steps);
+      if (is_hit) {
+        const uint32_t qid = a.L.entry_qid[v.y];  // only a hit needs its query
+        key = hit_key(a, qid, v.x, cpos - a.q_offsets[qid]);
+      }
+      n_steps += (uint32_t)steps;
+    }
+    __syncwarp();
+    hit.push(is_hit, key);
+    if (hit.n >= 32) hit.flush(a.hits, a.hit_count, a.hit_cap);
+  }
+};
+
+// Largest i in [lo, hi] with off[i] <= v (off non-decreasing, off[lo] <= v),
+// by the whole warp: 32 probes a round.
+__device__ __forceinline__ uint32_t warp_upper_segment(const uint64_t *off, uint32_t lo,
+                                                       uint32_t hi, uint64_t v) {
+  const uint32_t lane = threadIdx.x & 31;
+  while (lo < hi) {
+    const uint32_t step = (hi - lo) / 32 + 1;
+    const uint64_t i = lo + (uint64_t)(lane + 1) * step;
+    const unsigned m = __ballot_sync(0xffffffffu, i <= hi && off[i] <= v);
+    lo += (uint32_t)__popc(m) * step;
+    hi = min(hi, lo + step - 1);
+  }
+  return lo;
+}
+
+// Member work: (cluster, entry) of every passing representative.  Only
+// clusters with members are written; that is looked up here, 32 at a time,
+// rather than for every representative.
+struct MemberWork {
+  const SeedArgs &a;
+  WarpStack<uint2> stack;
+  __device__ __forceinline__ void add(bool have, uint32_t cid, uint32_t entry) {
+    stack.push(have, make_uint2(cid, entry));
+    if (stack.n >= 32) flush();
+  }
+  __device__ __forceinline__ void flush() {
+    const uint32_t lane = threadIdx.x & 31;
+    uint2 v = make_uint2(0, 0);
+    bool have = stack.pop(&v);
+    have = have && a.X.member_offsets[v.x + 1] > a.X.member_offsets[v.x];
+    const unsigned m = __ballot_sync(0xffffffffu, have);
+    unsigned long long base = 0;
+    if (lane == 0 && m) base = atomicAdd(a.mwork_count, (unsigned long long)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
+    if (have && base < a.mwork_cap) a.mwork[base] = v;
+  }
+  __device__ __forceinline__ void finish() {
+    if (stack.n) flush();
+  }
+};
+
 // One unit = one representative or one residual database position of a list,
-// tried against every query position of that list.  Bounded to six blocks
-// per SM (40 registers, a few spilled): the walks' global loads want the
-// warps more than the registers.
-__global__ void __launch_bounds__(kSeedBlock, 6)
+// tried against every query position of that list: the lanes take 32 units
+// and hand their seeds to the warp's walker, a list entry at a time.
+__global__ void __launch_bounds__(kSeedBlock, 3)
 seed_kernel(SeedArgs a) {
-  __shared__ __align__(16) int32_t tbl32[kWalkTableBytes / 4];
-  load_walk_table(tbl32, a.matrix32, a.p.delimiter);
-  __syncthreads();
-  const char *tbl = reinterpret_cast<const char *>(tbl32);
-  const int lane = threadIdx.x & 31;
+  __shared__ __align__(16) SeedShared sh;
+  SeedWalker walker(a, sh);
+  MemberWork mwork{a};
+  mwork.stack.item = sh.member[threadIdx.x >> 5];
+  const uint32_t lane = threadIdx.x & 31;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const uint64_t U = a.units_dev ? *a.units_dev : a.L.n_units;
-  const int thr = a.p.distance_threshold;
-  const int maxmd = a.p.max_member_distance;
-  // a thread's counts stay far below 2^32 (that many walk steps would take
-  // one thread seconds); 32-bit counters leave the six-block register
-  // budget to the walk
-  uint32_t n_dist = 0, n_seed = 0, n_steps = 0;
-  for (uint64_t base = warp * kUnitsPerWarp; base < U; base += nwarps * kUnitsPerWarp) {
-    const uint64_t last = min(base + kUnitsPerWarp, U) - 1;
-    // list range of this warp's units
-    uint64_t l_lo = 0, l_hi = 0;
-    if (lane == 0) {
-      l_lo = upper_segment(a.L.unit_offsets, 0, a.L.n_lists - 1, base);
-      l_hi = upper_segment(a.L.unit_offsets, l_lo, a.L.n_lists - 1, last);
-    }
-    l_lo = __shfl_sync(0xffffffffu, l_lo, 0);
-    l_hi = __shfl_sync(0xffffffffu, l_hi, 0);
-    for (uint64_t u = base + lane; u <= last; u += 32) {
-      const uint64_t l = upper_segment(a.L.unit_offsets, l_lo, l_hi, u);
-      const uint32_t j = (uint32_t)(u - a.L.unit_offsets[l]);
-      const uint32_t pb = a.L.offsets[l], pe = a.L.offsets[l + 1];
-      const uint32_t nchk = a.L.nchk[l];
-      const uint32_t nrep = a.L.rep_count[l];
-      if (j < nrep) {
-        // representative: distance filter for check positions
-        const uint32_t r = a.L.rep_begin[l] + j;
-        const uint32_t rpos = a.X.rep_positions[r];
-        const uint32_t cid = a.X.rep_cluster_ids[r];
-        const bool members = a.X.member_offsets[cid + 1] > a.X.member_offsets[cid];
-        const uint64_t rwin = a.X.rep_windows[r];
-        const uint8_t *dptr = a.db + rpos;
-        for (uint32_t k = pb; k < pe; ++k) {
-          const uint32_t cpos = a.L.entry_cpos[k];
-          const uint8_t *qptr = a.q + cpos;
-          bool try_rep, pass;
-          if (k < pb + nchk) {
+  constexpr uint32_t share = kUnitsPerWarp;
+  const int thr = a.p.distance_threshold, maxmd = a.p.max_member_distance;
+  uint32_t n_dist = 0;
+  for (uint64_t base = warp * share; base < U; base += nwarps * share) {
+    const uint64_t end = min(base + share, U);
+    uint32_t l = warp_upper_segment(a.L.unit_offsets, 0, (uint32_t)(a.L.n_lists - 1), base);
+    const uint32_t l_last =
+        warp_upper_segment(a.L.unit_offsets, l, (uint32_t)(a.L.n_lists - 1), end - 1);
+    for (uint64_t u0 = base; u0 < end; u0 += 32) {
+      const uint64_t u = u0 + lane;
+      uint32_t k = 0, pe = 0, chk_end = 0, d = 0, cid = 0;
+      uint64_t rwin = 0;
+      bool rep = false;
+      if (u < end) {
+        const uint64_t m = upper_segment(a.L.unit_offsets, l, l_last, u);
+        const uint32_t j = (uint32_t)(u - a.L.unit_offsets[m]);
+        k = a.L.offsets[m];
+        pe = a.L.offsets[m + 1];
+        const uint32_t nrep = a.L.rep_count[m];
+        rep = j < nrep;
+        if (rep) {
+          const uint32_t r = a.L.rep_begin[m] + j;
+          d = a.X.rep_positions[r];
+          cid = a.X.rep_cluster_ids[r];
+          rwin = a.X.rep_windows[r];
+          chk_end = k + a.L.nchk[m];
+        } else {
+          d = a.X.nc_values[a.L.nc_begin[m] + (j - nrep)];
+        }
+      }
+      while (__any_sync(0xffffffffu, k < pe)) {
+        bool have = k < pe, pass = have && rep;
+        uint32_t cpos = 0, ct = 0;
+        if (have) {
+          cpos = a.L.entry_cpos[k];
+          ct = a.L.entry_ct[k];
+          if (k < chk_end) {
             const int dist = nibble_mismatches(a.L.entry_window[k], rwin);
             ++n_dist;
-            try_rep = dist <= thr;
+            have = dist <= thr;
             pass = max(dist - maxmd, 0) <= thr;
-          } else {
-            try_rep = true;
-            pass = true;
           }
-          if (try_rep) {
-            int steps = 0;
-            ++n_seed;
-            const uint32_t ct = a.L.entry_ct[k];
-            if (walk_hit(qptr, dptr, tbl, (int)(ct >> 16), (int)(int16_t)(ct & 0xffffu),
-                         &steps)) {
-              const uint32_t qid = a.L.entry_qid[k];  // only a hit needs its query
-              emit_hit(a, qid, rpos, cpos - a.q_offsets[qid]);
-            }
-            n_steps += steps;
-          }
-          if (pass && members) append(a.mwork, a.mwork_count, a.mwork_cap, make_uint2(cid, k));
         }
-      } else {
-        const uint32_t d = a.X.nc_values[a.L.nc_begin[l] + (j - nrep)];
-        const uint8_t *dptr = a.db + d;
-        for (uint32_t k = pb; k < pe; ++k) {
-          const uint32_t cpos = a.L.entry_cpos[k];
-          int steps = 0;
-          ++n_seed;
-          const uint32_t ct = a.L.entry_ct[k];
-          if (walk_hit(a.q + cpos, dptr, tbl, (int)(ct >> 16), (int)(int16_t)(ct & 0xffffu),
-                       &steps)) {
-            const uint32_t qid = a.L.entry_qid[k];  // only a hit needs its query
-            emit_hit(a, qid, d, cpos - a.q_offsets[qid]);
-          }
-          n_steps += steps;
-        }
+        mwork.add(pass, cid, k);
+        walker.add(have, d, k, cpos, ct);
+        if (k < pe) ++k;
       }
     }
   }
-  __syncwarp();
+  walker.finish();
+  mwork.finish();
   add_counter(&a.ctr[0], n_dist);
-  add_counter(&a.ctr[1], n_seed);
-  add_counter(&a.ctr[2], n_steps);
+  add_counter(&a.ctr[1], walker.n_seed);
+  add_counter(&a.ctr[2], walker.n_steps);
 }
 
 // Members of a representative's cluster against one passing query position
@@ -542,27 +702,24 @@ seed_kernel(SeedArgs a) {
 // together, scans their member counts, and deals the (item, member) seeds
 // to its lanes 32 at a time: a lane finds its item with a five-step shuffle
 // search over the scan, so a seed costs one load (the member's position)
-// besides its walk.  Six blocks per SM, as seed_kernel.
-__global__ void __launch_bounds__(kSeedBlock, 6)
+// besides its walk.
+__global__ void __launch_bounds__(kSeedBlock, 3)
 member_kernel(SeedArgs a, const uint2 *__restrict__ mwork, uint64_t n_work,
               const uint64_t *n_dev) {
-  __shared__ __align__(16) int32_t tbl32[kWalkTableBytes / 4];
+  __shared__ __align__(16) SeedShared sh;
   if (n_dev) n_work = *n_dev;
-  load_walk_table(tbl32, a.matrix32, a.p.delimiter);
-  __syncthreads();
-  const char *tbl = reinterpret_cast<const char *>(tbl32);
+  SeedWalker walker(a, sh);
   const int lane = threadIdx.x & 31;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  uint32_t n_seed = 0, n_steps = 0;  // per thread, as in seed_kernel
   for (uint64_t i0 = warp * 32; i0 < n_work; i0 += nwarps * 32) {
     const uint64_t i = i0 + lane;
-    uint32_t mb = 0, cnt = 0, qid = 0, cpos = 0, ct = 0;
+    uint32_t mb = 0, cnt = 0, entry = 0, cpos = 0, ct = 0;
     if (i < n_work) {
       const uint2 mw = mwork[i];
       mb = a.X.member_offsets[mw.x];
       cnt = a.X.member_offsets[mw.x + 1] - mb;
-      qid = a.L.entry_qid[mw.y];
+      entry = mw.y;
       cpos = a.L.entry_cpos[mw.y];
       ct = a.L.entry_ct[mw.y];
     }
@@ -579,27 +736,19 @@ member_kernel(SeedArgs a, const uint2 *__restrict__ mwork, uint64_t n_work,
       // inclusive offset, since every later lane starts beyond p)
       int o = 0;
       for (int step = 16; step >= 1; step >>= 1) {
-        const uint32_t e = __shfl_sync(0xffffffffu, excl, o + step);
+        const uint32_t e = __shfl_sync(0xffffffffu, excl, (o + step) & 31);
         if (o + step < 32 && e <= p) o += step;
       }
       const uint32_t m = __shfl_sync(0xffffffffu, mb, o) + (p - __shfl_sync(0xffffffffu, excl, o));
-      const uint32_t sq = __shfl_sync(0xffffffffu, qid, o);
+      const uint32_t se = __shfl_sync(0xffffffffu, entry, o);
       const uint32_t sc = __shfl_sync(0xffffffffu, cpos, o);
-      const uint32_t sct = __shfl_sync(0xffffffffu, ct, o);
-      if (p < total) {
-        const uint32_t d = a.X.member_positions[m];
-        int steps = 0;
-        ++n_seed;
-        if (walk_hit(a.q + sc, a.db + d, tbl, (int)(sct >> 16), (int)(int16_t)(sct & 0xffffu),
-                     &steps))
-          emit_hit(a, sq, d, sc - a.q_offsets[sq]);
-        n_steps += steps;
-      }
+      const uint32_t st = __shfl_sync(0xffffffffu, ct, o);
+      walker.add(p < total, p < total ? a.X.member_positions[m] : 0, se, sc, st);
     }
   }
-  __syncwarp();
-  add_counter(&a.ctr[1], n_seed);
-  add_counter(&a.ctr[2], n_steps);
+  walker.finish();
+  add_counter(&a.ctr[1], walker.n_seed);
+  add_counter(&a.ctr[2], walker.n_steps);
 }
 
 // ---------------------------------------------------------------------------
@@ -2558,8 +2707,8 @@ int presearch_impl(gzb_engine *e, int schedule, cudaStream_t s) {
                             e->mwork_alt.as<uint64_t>(), n_mwork, bits_for(X.n_reps + 1), s,
                             &sorted_mw));
       launches += 1;
-      member_kernel<<<grid1((n_mwork + 31) / 32 * 32, kSeedBlock, 148 * 16), kSeedBlock, 0, s>>>(
-          a, reinterpret_cast<const uint2 *>(sorted_mw), n_mwork, nullptr);
+      member_kernel<<<grid1((n_mwork + 31) / 32 * 32, kSeedBlock, 148 * 16), kSeedBlock, 0,
+                      s>>>(a, reinterpret_cast<const uint2 *>(sorted_mw), n_mwork, nullptr);
       GZB_CUDA(cudaGetLastError());
       ++launches;
       GZB_CUDA(cudaMemcpyAsync(hctr, c, 64, cudaMemcpyDeviceToHost, s));
@@ -2962,8 +3111,8 @@ int graph_body(gzb_engine *e, int schedule, const GappedTile &tile, bool learned
   GZB_TRY(sort_keys_u64(e, reinterpret_cast<uint64_t *>(a.mwork), e->mwork_alt.as<uint64_t>(),
                         c.mwork, bits_for(X.n_reps + 1), s, &sorted_mw));
   ++launches;
-  member_kernel<<<148 * 16, kSeedBlock, 0, s>>>(a, reinterpret_cast<const uint2 *>(sorted_mw),
-                                                c.mwork, plan + 0);
+  member_kernel<<<148 * 16, kSeedBlock, 0, s>>>(
+      a, reinterpret_cast<const uint2 *>(sorted_mw), c.mwork, plan + 0);
   GZB_CUDA(cudaGetLastError());
   ++launches;
   stamp_kernel<<<1, 1, 0, s>>>(plan + 24 + 6);

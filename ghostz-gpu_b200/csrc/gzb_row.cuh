@@ -151,13 +151,13 @@ __host__ __device__ __forceinline__ void row_store4(uint32_t a, const RowGroup &
 #endif
 }
 // a score-table entry (the table does not change)
-__host__ __device__ __forceinline__ int row_entry(uint32_t a) {
+__host__ __device__ __forceinline__ uint32_t row_load_const(uint32_t a) {
 #ifdef __CUDA_ARCH__
-  int v;
-  asm("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a));
+  uint32_t v;
+  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
   return v;
 #else
-  return *reinterpret_cast<int *>(row_host_memory + a);
+  return *reinterpret_cast<uint32_t *>(row_host_memory + a);
 #endif
 }
 // byte j of w, plus a
@@ -421,8 +421,8 @@ __host__ __device__ __forceinline__ int row_step(const GappedJob &job, uint32_t 
     do {
       const RowGroup w = cur;
       const int sc[4] = {
-          row_entry(row_byte_plus<0>(res, row)), row_entry(row_byte_plus<1>(res, row)),
-          row_entry(row_byte_plus<2>(res, row)), row_entry(row_byte_plus<3>(res, row))};
+          (int)row_load_const(row_byte_plus<0>(res, row)), (int)row_load_const(row_byte_plus<1>(res, row)),
+          (int)row_load_const(row_byte_plus<2>(res, row)), (int)row_load_const(row_byte_plus<3>(res, row))};
       cur = row_load4(band.group(g + 1));
       res = row_load(band.residues(g + 1));
       if (flags != 15) {

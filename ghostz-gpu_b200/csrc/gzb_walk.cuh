@@ -1,0 +1,164 @@
+// gzb_walk.cuh -- the ungapped X-drop extension of a seed over a window of
+// 32 residues either side, without branches (the seed search's first pass).
+//
+// SeedSearcher::UngappedExtend (src/seed_searcher.h:133-158) walks from the
+// seed both ways until the score falls `cutoff` below its best or a
+// delimiter is met, and asks whether the two bests sum to more than
+// `trigger`.  Nine walks in ten end within 32 pairs on either side, and
+// 987 seeds in 1,000 stay far below the trigger.  walk_window evaluates
+// 32 pairs of both sides for every seed: where both walks end and even the
+// windows' largest scores (an upper bound of the bests) do not exceed the
+// trigger, the seed is settled, with the exact number of pairs the walks
+// examined; the other seeds are left to walk_hit, 32 of them together.
+//
+// Both sides are computed in one word, reverse in the low half and forward in
+// the high half, scores doubled.  Per pair of pairs: two table words (the
+// forward table's entries are << 16), score, running best, drop below it,
+// and a sticky flag whose sum counts the steps from the walk's end on.  A
+// delimiter's entry is odd, so that bit 0 of the drop tells a walk that a
+// delimiter ended.  Exact for matrix entries up to kWalkMaxEntry in size and
+// cutoffs 1 .. kWalkMaxCutoff.
+//
+// The 64 bytes around a position are read as three aligned 32-byte words: a
+// scattered request costs the L1 cache one cycle per lane's 32-byte sector
+// that misses, and at least ten a request whatever its width.  Measured on a
+// B200, 32 random windows of an L2-resident chunk an SM: 97 cycles (three
+// 32-byte loads a lane), 114 (five 16-byte loads), 161 (not allocated in
+// L1); twenty 4-byte loads cost ten cycles each even where all hit.
+#pragma once
+
+#include <cstdint>
+
+#include "gzb_kernels.cuh"
+#include "gzb_row.cuh"
+
+namespace gzb {
+
+constexpr int kWindow = 32;           // residue pairs either side
+constexpr int kWalkMaxEntry = 127;
+constexpr int kWalkMaxCutoff = 127;
+constexpr int kWalkStop = -513;       // a delimiter's (doubled) entry
+constexpr int kWalkBias = 0x5000;     // keeps a half from borrowing
+constexpr int kWalkFlag = 0x400;      // set in a drop of at least cutoff
+
+// Score table: the doubled score of (query code a, database code b) at byte
+// 256 a + 4 (a ^ b) (reverse) and, << 16, 128 bytes behind (forward).  The
+// XOR puts pairs that share a code into different banks.
+constexpr int kWindowTableBytes = 32 * 256;
+
+__host__ __device__ __forceinline__ int window_entry(int a, int b, int score, int delim) {
+  return a == delim || b == delim ? kWalkStop : 2 * score;
+}
+
+// Fills the table; returns (on every thread) whether the matrix is admitted.
+__device__ __forceinline__ bool load_window_table(uint32_t tbl, const int32_t *m32, int delim) {
+  bool fits = true;
+  for (int i = threadIdx.x; i < 32 * 32; i += blockDim.x) {
+    const int a = i >> 5, x = i & 31, b = a ^ x;
+    const int score = m32[b * 32 + a];
+    fits = fits && score >= -kWalkMaxEntry && score <= kWalkMaxEntry;
+    const int v = window_entry(a, b, score, delim);
+    row_store(tbl + 256 * a + 4 * x, (uint32_t)v);
+    row_store(tbl + 256 * a + 4 * x + 128, (uint32_t)v << 16);
+  }
+  return __syncthreads_and(fits) != 0;
+}
+
+// The 32-byte words that hold s[-32 .. 31] (between s - 63 and s + 63).
+struct WindowWords {
+  uint32_t w[24];
+};
+
+__host__ __device__ __forceinline__ void fetch_window(const uint8_t *s, WindowWords &ww) {
+  const uintptr_t p = (uintptr_t)s;
+  const uintptr_t start = (p - kWindow) & ~(uintptr_t)31;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+#ifdef __CUDA_ARCH__
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(ww.w[8 * i]), "=r"(ww.w[8 * i + 1]), "=r"(ww.w[8 * i + 2]),
+          "=r"(ww.w[8 * i + 3]), "=r"(ww.w[8 * i + 4]), "=r"(ww.w[8 * i + 5]),
+          "=r"(ww.w[8 * i + 6]), "=r"(ww.w[8 * i + 7])
+        : "l"(start + 32 * i));
+#else
+    for (int j = 0; j < 8; ++j) ww.w[8 * i + j] = reinterpret_cast<const uint32_t *>(start)[8 * i + j];
+#endif
+  }
+}
+
+// The residues s[-32 .. 31] of the fetched words, four a word.
+__host__ __device__ __forceinline__ void align_window(const uint8_t *s, const WindowWords &ww,
+                                                      uint32_t a[16]) {
+  const uint32_t p = (uint32_t)(uintptr_t)s;
+  const int shift = 8 * (int)(p & 3);
+  const uint32_t start = p - kWindow;
+  const bool by4 = (start & 16) != 0, by2 = (start & 8) != 0, by1 = (start & 4) != 0;
+  uint32_t w[20];
+#pragma unroll
+  for (int i = 0; i < 20; ++i) w[i] = by4 ? ww.w[i + 4] : ww.w[i];
+#pragma unroll
+  for (int i = 0; i < 18; ++i) w[i] = by2 ? w[i + 2] : w[i];
+#pragma unroll
+  for (int i = 0; i < 17; ++i) w[i] = by1 ? w[i + 1] : w[i];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) a[i] = row_funnel_r(w[i], w[i + 1], shift);
+}
+
+// byte J of x | byte J of a << 8 (x below 128: its sign bit fills the rest)
+template <int J>
+__host__ __device__ __forceinline__ uint32_t window_offset(uint32_t x, uint32_t a) {
+#ifdef __CUDA_ARCH__
+  return walk_offset<J>(x, a);
+#else
+  return ((x >> (8 * J)) & 0xffu) | (((a >> (8 * J)) & 0xffu) << 8);
+#endif
+}
+
+__host__ __device__ __forceinline__ uint32_t window_addmax(uint32_t a, uint32_t b, uint32_t c) {
+#ifdef __CUDA_ARCH__
+  return __viaddmax_u16x2(a, b, c);  // per half max(a + b, c)
+#else
+  const uint32_t lo = ((a & 0xffffu) + (b & 0xffffu)) & 0xffffu, hi = ((a >> 16) + (b >> 16)) & 0xffffu;
+  const uint32_t cl = c & 0xffffu, ch = c >> 16;
+  return (lo > cl ? lo : cl) | ((hi > ch ? hi : ch) << 16);
+#endif
+}
+
+// Whether the seed is settled as no hit; *steps then holds the residue pairs
+// its two walks examine.
+__host__ __device__ __forceinline__ bool walk_window(uint32_t tbl, const uint32_t q[16],
+                                                     const uint32_t d[16], int cutoff,
+                                                     int trigger, int *steps) {
+  const uint32_t add = 0x10001u * (uint32_t)(kWalkFlag - 2 * cutoff);
+  uint32_t score = 0x10001u * kWalkBias;
+  uint32_t best = score + add;  // best + add
+  uint32_t flags = 0, sum = 0;
+#define GZB_WINDOW_PAIR(J)                                                       \
+  {                                                                              \
+    const uint32_t r = row_load_const(tbl + window_offset<3 - (J)>(xr, q[7 - k])); \
+    const uint32_t f = row_load_const(tbl + window_offset<(J)>(xf, q[8 + k]) + 128); \
+    score = score + r + f;                                                       \
+    best = window_addmax(score, add, best);                                      \
+    flags = (flags | (best - score)) & (0x10001u * (kWalkFlag | 1));             \
+    sum += flags;                                                                \
+  }
+#pragma unroll
+  for (int k = 0; k < kWindow / 4; ++k) {
+    const uint32_t xr = (q[7 - k] ^ d[7 - k]) << 2, xf = (q[8 + k] ^ d[8 + k]) << 2;
+    GZB_WINDOW_PAIR(0)
+    GZB_WINDOW_PAIR(1)
+    GZB_WINDOW_PAIR(2)
+    GZB_WINDOW_PAIR(3)
+  }
+#undef GZB_WINDOW_PAIR
+  // steps from the end on (0: the walk goes on), and of those that a
+  // delimiter had been met
+  const int nr = (int)(sum & 0xffffu) / kWalkFlag, nf = (int)(sum >> 16) / kWalkFlag;
+  const int zr = (int)(sum & (kWalkFlag - 1)), zf = (int)((sum >> 16) & (kWalkFlag - 1));
+  const int bests = (int)(best & 0xffffu) + (int)(best >> 16) -
+                    2 * (int)((add & 0xffffu) + kWalkBias);
+  *steps = 2 * (kWindow + 1) - nr - nf - (zr == nr ? 1 : 0) - (zf == nf ? 1 : 0);
+  return nr > 0 && nf > 0 && bests <= 2 * trigger;
+}
+
+}  // namespace gzb
