@@ -12,11 +12,7 @@
 //
 // The warp evaluates 32 consecutive columns of a row at once, with the
 // presearch's warp DP (gapped_extend_warp in gzb_kernels.cuh: band edges and
-// stored values exact for X-drops below 1024).  A kept cell's edit op also
-// needs the reference's horizontal-gap value *with* its reset to
-// kInitScore at pruned cells (src/gapped_extender.cpp:428-446); once a
-// chunk's pruned flags are known that value is a segmented max-plus scan
-// whose segments start after the pruned cells.  Sides whose band outgrows
+// stored values exact for X-drops below 1024).  Sides whose band outgrows
 // the warp's circular buffer, whose storage outgrows the warp's scratch, or
 // whose X-drop is 1024 or more are flagged and run by one thread each: a
 // pass to size their storage, then the DP with the band in global memory
@@ -200,25 +196,52 @@ __device__ void tb_extend(const TbArgs &a, const int *sm, const TbSide &t, int2 
 }
 
 constexpr int kTbWarpColumns = 256;  // circular band of one warp (int2 columns)
+constexpr int kTbMaxBand = kTbWarpColumns - 32;  // (residues are read 32 columns ahead)
 constexpr int kTbWarpsPerBlock = 8;
 static_assert(kTbWarpBlock == kTbWarpsPerBlock * 32, "launch block of the warp kernels");
 
-// tb_extend by one warp (lanes must all call it with the same side); with
-// STORE it also writes the ops and row table as tb_extend does, into
-// storage of ops_cap bytes and rows_cap rows that need not be zeroed: every
-// byte of a row's range is written (0 for a pruned cell and the sentinel,
-// as a fresh GappedExtender holds), and the bytes past the last row up to
-// *ops_bytes are zeroed at the end.  Returns false when the band outgrows
-// kTbWarpColumns or the side outgrows the storage (outputs then
-// meaningless).
-template <bool STORE>
-__device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, int2 *band,
+// A warp's band: the cells and the query residues of its columns.
+struct TbBand {
+  int2 cell[kTbWarpColumns];
+  uint8_t res[kTbWarpColumns];
+};
+
+// tb_extend by one warp (lanes must all call it with the same side); it
+// also writes the ops and row table as tb_extend does, into storage of
+// ops_cap bytes and rows_cap rows that need not be zeroed: every byte of a
+// row's range is written (0 for a pruned cell and the sentinel, as a fresh
+// GappedExtender holds), and the bytes past the last row up to *ops_bytes
+// are zeroed at the end.  Returns false when the band outgrows kTbMaxBand or
+// the side outgrows the storage (outputs then meaningless).
+//
+// A row's latency is what long sides wait for and its instructions are what
+// many short ones cost, so a chunk of 32 columns runs only the scans that can
+// change something:
+//  * the horizontal gap's scan where a gap could be alive at all: one comes
+//    in at or above the threshold t = max - X-drop, or some cell could open
+//    one (score - gap >= t).  Gaps below t keep no cell, start no path
+//    operation and grow no band.
+//  * the running maximum's scan where a cell exceeds it.
+// The gap is not reset behind a pruned cell, for the ops as for the
+// decisions: where that differs from the reference's, the gap is below t.  A
+// kept cell's score is not, so its op is the same; an extension flag is read
+// on the path only behind a gap at or above t, which came from the cell's
+// score, so the flag is clear either way.
+// No load of a row depends on its scores: the next database residue is
+// fetched a row ahead, the query's residues and its delimiter's column 32
+// columns ahead.
+// All scans of every chunk, and the loads where their values were needed,
+// took (the whole kernel) 4.2 ms on the alignments of 1,000 queries x 20,000
+// proteins, which long homologs dominate, and 18.7 ms on those of 30,000
+// reads x 400,000; this takes 3.2 and 14.0 ms.
+__device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, TbBand &band,
                                uint8_t *ops, uint32_t *row_meta, uint64_t ops_cap,
                                uint32_t rows_cap, uint64_t *ops_bytes, uint32_t *rows,
                                int *best_score, int *best_p0, int *best_p1) {
-  constexpr int W = kTbWarpColumns;
-  constexpr int wmask = W - 1;
+  constexpr int W = kTbMaxBand;
+  constexpr int wmask = kTbWarpColumns - 1;
   constexpr unsigned full = 0xffffffffu;
+  constexpr int kFar = 1 << 30;
   const int lane = threadIdx.x & 31;
   const int inc = t.inc;
   const int delim = a.delim;
@@ -231,31 +254,41 @@ __device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, 
   *best_p1 = -inc;
   *ops_bytes = 0;
   *rows = 0;
-  if (q0[0] == delim || d0[0] == delim) return true;
+  int x = d0[0];
+  if (q0[0] == delim || x == delim) return true;
+  // columns 1 .. seen have their residues in the band; the query's delimiter
+  // is at column delim_at (kFar: not seen).  Up to 32 columns past the
+  // delimiter are read (the sequences are padded).
+  int seen = 0, delim_at = kFar;
+  auto see = [&](int c) {  // the columns up to c (or the delimiter's)
+    while (seen < c && delim_at == kFar) {
+      const int k = seen + 1 + lane;
+      const int r = q0[(k - 1) * inc];
+      band.res[k & wmask] = (uint8_t)r;
+      const unsigned m = __ballot_sync(full, r == delim);
+      if (m) delim_at = seen + __ffs(m);
+      seen += 32;
+    }
+  };
   // row -1: the horizontal gap run from column 1 while >= -cutoff
-  int k0;
-  if (-gi < -cutoff) {
-    k0 = 0;
-  } else if (ge == 0) {
-    k0 = 1 << 30;
-  } else {
-    const long long kk = ((long long)cutoff - gi) / ge + 1;
-    k0 = kk > (1 << 30) ? (1 << 30) : (int)kk;
+  int k0 = 0;
+  if (cutoff >= gi) {
+    const long long kk = ge == 0 ? kFar : ((long long)cutoff - gi) / ge + 1;
+    k0 = kk > kFar ? kFar : (int)kk;
   }
-  int col = find_delimiter_column(q0, inc, delim, 1, k0 > W ? W + 1 : k0);
+  see(imin(k0, W) + 1);
+  const int col = imin(k0 + 1, delim_at);
   if (col > W) return false;
   for (int c = 1 + lane; c < col; c += 32) {
     const int s = -gi - (c - 1) * ge;
-    band[c & wmask] = make_int2(s, s - gi);
+    band.cell[c & wmask] = make_int2(s, s - gi);
   }
-  if (lane == 0) band[0] = make_int2(0, -gi);
-  int bs = 0, be;
-  if (q0[(col - 1) * inc] != delim) {
+  if (lane == 0) band.cell[0] = make_int2(0, -gi);
+  int bs = 0, be = col;
+  if (col < delim_at) {
     if (col + 1 > W) return false;
-    if (lane == 0) band[col & wmask] = make_int2(kInitScore, kInitScore);
+    if (lane == 0) band.cell[col & wmask] = make_int2(kInitScore, kInitScore);
     be = col + 1;
-  } else {
-    be = col;
   }
   __syncwarp();
 
@@ -264,34 +297,29 @@ __device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, 
   uint64_t written = 0;  // end of the bytes the rows wrote
   uint32_t r = 0;
   for (;; ++r) {
-    const int x = d0[(int)r * inc];
     if (x == delim) break;
     const int *mrow = sm + x * kMatrixStride;
+    x = d0[((int)r + 1) * inc];
     const int row_start = bs;
-    uint8_t *row_ops = nullptr;
-    if (STORE) {
-      // a row's storage runs from its first band column to the next row's
-      // band end: at most 2 W + 1 columns (the band, W wide, may move right
-      // by up to W within the row), and the sentinel
-      if (used + 2 * W + 2 > ops_cap || r >= rows_cap) return false;
-      if (lane == 0) {
-        row_meta[2 * r] = (uint32_t)used;
-        row_meta[2 * r + 1] = (uint32_t)row_start;
-      }
-      row_ops = ops + used - row_start;
+    // a row's storage runs from its first band column to the next row's band
+    // end: at most 2 W + 1 columns (the band, W wide, may move right by up
+    // to W within the row), and the sentinel
+    if (used + 2 * W + 2 > ops_cap || r >= rows_cap) return false;
+    if (lane == 0) {
+      row_meta[2 * r] = (uint32_t)used;
+      row_meta[2 * r + 1] = (uint32_t)row_start;
     }
+    uint8_t *row_ops = ops + used - row_start;
     // column bs: vertical gap only
-    const int2 st0 = band[bs & wmask];
+    const int2 st0 = band.cell[bs & wmask];
     int diag = st0.x;
     const int nb0 = (maxs - st0.y > cutoff) ? kInitScore : st0.y;
-    int F = nb0 - gi;   // horizontal gap without the reset at pruned cells
-    int Fs = nb0 - gi;  // the reference's horizontal gap
+    int F = nb0 - gi;  // the horizontal gap entering the chunk
     __syncwarp();
     if (lane == 0) {
-      band[bs & wmask] = make_int2(nb0, st0.y - ge);
-      if (STORE) row_ops[bs] = kTbGap0 + kTbExt0;
+      band.cell[bs & wmask] = make_int2(nb0, st0.y - ge);
+      row_ops[bs] = kTbGap0 + kTbExt0;
     }
-    int M = maxs;
     int first_kept = -1, last_kept = bs;
     for (int cs = bs + 1; cs < be; cs += 32) {
       const int c = cs + lane;
@@ -299,91 +327,65 @@ __device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, 
       int2 st = make_int2(kInitScore, kInitScore);
       int qres = 0;
       if (active) {
-        st = band[c & wmask];
-        qres = q0[(c - 1) * inc];
+        st = band.cell[c & wmask];
+        qres = band.res[c & wmask];
       }
       int prev = __shfl_up_sync(full, st.x, 1);
       if (lane == 0) prev = diag;
       const int sd = prev + mrow[qres];
       const int G = imax(sd, st.y);
-      int P = active ? G - gi + (lane + 1) * ge : kNegBig;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int tv = __shfl_up_sync(full, P, o);
-        if (lane >= o) P = imax(P, tv);
-      }
-      int Pex = __shfl_up_sync(full, P, 1);
-      if (lane == 0) Pex = kNegBig;
-      const int raw = imax(G, imax(F, Pex) - lane * ge);
-      int R = active ? raw : kNegBig;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int tv = __shfl_up_sync(full, R, o);
-        if (lane >= o) R = imax(R, tv);
-      }
-      const int Mrow = imax(M, R);
-      const bool pruned = (Mrow - raw > cutoff);
-      if (active) {
-        const int nb = pruned ? kInitScore : raw;
-        const int ng = pruned ? kInitScore : imax(raw - gi, st.y - ge);
-        band[c & wmask] = make_int2(nb, ng);
-      }
       const int nact = imin(32, be - cs);
-      if (STORE) {
-        // the reference's horizontal gap entering each cell: normalized
-        // N(j) = F(j) + j ge obeys N(j + 1) = max(N(j), G(j) - gi + (j + 1) ge)
-        // after a kept cell and restarts at kInitScore + (j + 1) ge after a
-        // pruned one (a segment head)
-        const bool head = active && pruned;
-        int v = head ? kInitScore + (lane + 1) * ge : (active ? G - gi + (lane + 1) * ge : kNegBig);
-        if (lane == 0 && !head) v = imax(v, Fs);
-        bool seg = head;
+      const int thr = maxs - cutoff;
+      int Fl = kNegBig;  // the horizontal gap entering the cell
+      if (F >= thr || __any_sync(full, active && G - gi >= thr)) {
+        int P = active ? G - gi + (lane + 1) * ge : kNegBig;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-          const int tv = __shfl_up_sync(full, v, o);
-          const bool ts = __shfl_up_sync(full, seg, o);
-          if (lane >= o) {
-            if (!seg) v = imax(v, tv);
-            seg = seg || ts;
-          }
+          const int tv = __shfl_up_sync(full, P, o);
+          if (lane >= o) P = imax(P, tv);
         }
-        int Nin = __shfl_up_sync(full, v, 1);
-        if (lane == 0) Nin = Fs;
-        if (active && pruned) row_ops[c] = 0;
-        if (active && !pruned) {
-          const int Fb = Nin - lane * ge;
-          int op = kTbSub, sc = sd;
-          if (sc < st.y) {
-            op = kTbGap0;
-            sc = st.y;
-          }
-          if (sc < Fb) {
-            op = kTbGap1;
-            sc = Fb;
-          }
-          if (!(st.y - ge < sc - gi)) op += kTbExt0;
-          if (!(Fb - ge < sc - gi)) op += kTbExt1;
-          row_ops[c] = (uint8_t)op;
-        }
-        Fs = __shfl_sync(full, v, nact - 1) - nact * ge;
+        int Pex = __shfl_up_sync(full, P, 1);
+        if (lane == 0) Pex = kNegBig;
+        Fl = imax(F, Pex) - lane * ge;
+        F = imax(F, __shfl_sync(full, P, nact - 1)) - nact * ge;
+      } else {
+        F = kNegBig;
       }
-      // new maximum: first column reaching the chunk maximum
-      const int cm = __shfl_sync(full, R, 31);
-      if (cm > M) {
-        const unsigned hitm = __ballot_sync(full, active && raw == cm);
-        const int l = __ffs(hitm) - 1;
-        maxs = cm;
-        mp0 = (cs + l - 1) * inc;
+      const int raw = imax(G, Fl);
+      int Mrow = maxs;
+      if (__any_sync(full, active && raw > maxs)) {
+        int R = active ? raw : kNegBig;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int tv = __shfl_up_sync(full, R, o);
+          if (lane >= o) R = imax(R, tv);
+        }
+        Mrow = imax(maxs, R);
+        // the new maximum: first column reaching it
+        maxs = __shfl_sync(full, R, 31);
+        const unsigned hitm = __ballot_sync(full, active && raw == maxs);
+        mp0 = (cs + __ffs(hitm) - 2) * inc;
         mp1 = (int)r * inc;
       }
-      const unsigned kept = __ballot_sync(full, active && !pruned);
+      const bool keep = active && Mrow - raw <= cutoff;
+      if (active) {
+        const int ng = imax(raw - gi, st.y - ge);
+        band.cell[c & wmask] =
+            keep ? make_int2(raw, ng) : make_int2(kInitScore, kInitScore);
+        int op = 0;
+        if (keep) {
+          op = sd < st.y ? kTbGap0 : kTbSub;
+          if (G < Fl) op = kTbGap1;
+          if (st.y - ge >= raw - gi) op += kTbExt0;
+          if (Fl - ge >= raw - gi) op += kTbExt1;
+        }
+        row_ops[c] = (uint8_t)op;
+      }
+      const unsigned kept = __ballot_sync(full, keep);
       if (kept) {
         if (first_kept < 0) first_kept = cs + __ffs(kept) - 1;
         last_kept = cs + 31 - __clz(kept);
       }
-      const int Plast = __shfl_sync(full, P, nact - 1);
-      F = imax(F, Plast) - nact * ge;
-      M = imax(M, cm);
       diag = __shfl_sync(full, st.x, 31);
     }
     __syncwarp();
@@ -393,39 +395,33 @@ __device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, 
       break;
     }
     bs = first_kept - 1;
-    bool edge_residue;
+    int edge = be;  // the column whose residue the reference tests
     if (last_kept < be - 1) {
-      edge_residue = q0[(be - 1) * inc] != delim;
       be = last_kept + 1;
     } else {
-      int k;
+      // grow along the horizontal gap while F >= max - cutoff
       const long long room = (long long)F - ((long long)maxs - cutoff);
-      if (room < 0) {
-        k = 0;
-      } else if (ge == 0) {
-        k = 1 << 30;
-      } else {
-        const long long kk = room / ge + 1;
-        k = kk > (1 << 30) ? (1 << 30) : (int)kk;
-      }
-      if (k > 0) {
-        const int lim = (be + k - bs > W) ? (W - (be - bs) + 1) : k;
-        k = find_delimiter_column(q0, inc, delim, be, lim) - be;
+      if (room >= 0) {
+        const long long kk = ge == 0 ? kFar : room / ge + 1;
+        const int k1 = (int)(kk > kFar ? kFar : kk);
+        see(be + imin(k1, W));
+        const int k = imin(k1, delim_at - be);
         if (be + k - bs > W) return false;
         for (int j = lane; j < k; j += 32) {
           const int v = F - j * ge;
-          band[(be + j) & wmask] = make_int2(v, v - gi);
-          if (STORE) row_ops[be + j] = kTbGap0 + kTbExt0;
+          band.cell[(be + j) & wmask] = make_int2(v, v - gi);
+          row_ops[be + j] = kTbGap0 + kTbExt0;
         }
         be += k;
       }
-      edge_residue = q0[(be - 1) * inc] != delim;
+      edge = be;
     }
-    if (edge_residue) {
+    see(edge);
+    if (edge < delim_at) {
       if (be + 1 - bs > W) return false;
       if (lane == 0) {
-        band[be & wmask] = make_int2(kInitScore, kInitScore);
-        if (STORE) row_ops[be] = 0;  // the sentinel
+        band.cell[be & wmask] = make_int2(kInitScore, kInitScore);
+        row_ops[be] = 0;  // the sentinel
       }
       ++be;
     }
@@ -434,12 +430,10 @@ __device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, 
     __syncwarp();
   }
   *ops_bytes = used + (uint64_t)(t.len0 + 2);
-  if (STORE) {
-    // past the rows: zeros up to the storage the reference would keep
-    if (*ops_bytes > ops_cap) return false;
-    for (uint64_t j = written + lane; j < *ops_bytes; j += 32) ops[j] = 0;
-    __syncwarp();
-  }
+  // past the rows: zeros up to the storage the reference would keep
+  if (*ops_bytes > ops_cap) return false;
+  for (uint64_t j = written + lane; j < *ops_bytes; j += 32) ops[j] = 0;
+  __syncwarp();
   *rows = r;
   *best_score = maxs;
   *best_p0 = mp0;
@@ -538,7 +532,7 @@ __device__ TbStats tb_walk_stats(const uint8_t *ops, const uint32_t *meta, int i
 // sides gather; then each lane walks one of them (PickOptimalPath and
 // BuildResult's counts), the 32 walks in parallel, and the scratch is
 // reused.  A side the warp cannot run exactly (X-drop >= 1024, a band wider
-// than kTbWarpColumns) or whose storage outgrows an empty scratch is
+// than kTbMaxBand) or whose storage outgrows an empty scratch is
 // flagged in `redo` with its sizes left to the thread kernels; the others
 // get zero sizes.
 __global__ void __launch_bounds__(kTbWarpsPerBlock * 32, 4)
@@ -546,7 +540,7 @@ __global__ void __launch_bounds__(kTbWarpsPerBlock * 32, 4)
                         int32_t *side_p0, int32_t *side_p1, TbStats *stats, uint64_t *ops_bytes,
                         uint64_t *rows, uint8_t *redo) {
   __shared__ int sm[kMatrixStride * kMatrixStride];
-  __shared__ int2 bands[kTbWarpsPerBlock][kTbWarpColumns];
+  __shared__ TbBand bands[kTbWarpsPerBlock];
   load_matrix(sm, a.matrix32, 32, 32);  // the 32 x 32 device matrix
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -585,7 +579,7 @@ __global__ void __launch_bounds__(kTbWarpsPerBlock * 32, 4)
         uint64_t nb;
         uint32_t nr;
         int sc, p0, p1;
-        ok = tb_extend_warp<true>(a, sm, t, bands[warp], ops_arena + ops_pos,
+        ok = tb_extend_warp(a, sm, t, bands[warp], ops_arena + ops_pos,
                                   meta_arena + 2 * (uint64_t)meta_pos, kTbScratchOps - ops_pos,
                                   kTbScratchRows - meta_pos, &nb, &nr, &sc, &p0, &p1);
         if (ok) {
