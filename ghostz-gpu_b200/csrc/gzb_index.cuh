@@ -89,10 +89,27 @@ __device__ __forceinline__ uint64_t pack_window(const DevParams &p, const uint8_
   return w;
 }
 
+// A window's nibbles as two words, the low two bits of each and the high two
+// (nibble t of the low half at bits 4t, of the high half at 4t + 2): what
+// many windows are compared with is laid out once, and a comparison is then
+// five operations and a population count.
+struct NibblePlanes {
+  uint32_t low, high;
+};
+
+__device__ __forceinline__ NibblePlanes nibble_planes(uint64_t w) {
+  const uint32_t lo = (uint32_t)w, hi = (uint32_t)(w >> 32);
+  return {(lo & 0x33333333u) | ((hi << 2) & 0xccccccccu),
+          ((lo >> 2) & 0x33333333u) | (hi & 0xccccccccu)};
+}
+
+__device__ __forceinline__ int plane_mismatches(NibblePlanes a, NibblePlanes b) {
+  const uint32_t x = (a.low ^ b.low) | (a.high ^ b.high);
+  return __popc((x | (x >> 1)) & 0x55555555u);
+}
+
 __device__ __forceinline__ int nibble_mismatches(uint64_t a, uint64_t b) {
-  uint64_t x = a ^ b;
-  x = (x | (x >> 1) | (x >> 2) | (x >> 3)) & 0x1111111111111111ull;
-  return __popcll(x);
+  return plane_mismatches(nibble_planes(a ^ b), {0, 0});
 }
 
 // Binary search in a sorted key array; returns index or -1.
