@@ -9,15 +9,15 @@
 // ungapped X-drop and the gapped-extension trigger
 // (src/aligner_gpu.cpp:228-238, src/statistics.cpp:28-43).
 //
-// One warp per query, in two passes (buffers for 24 rounds of the K series,
-// then for all 100 for the rare query that needs more).  The composition is
-// counted by the whole warp; the
-// score distribution's j-fold convolutions for K are spread over the lanes
-// (each lane owns whole entries, so every entry is summed in the
-// reference's order); every serial sum stays on lane 0 in the reference's
-// order.  All arithmetic uses explicitly rounded operations (no fused
-// multiply-add), so the float results agree with the reference's x86-64
-// build bit for bit; exp, pow and log are CUDA's double-precision functions.
+// Few queries take a warp each (karlin_kernel: the score distribution's
+// j-fold convolutions for K are spread over the lanes, the serial sums stay
+// on lane 0), many four lanes each (karlin_group_kernel).  Both first run
+// with buffers for the rounds of the K series that nearly every query needs;
+// one that needs more is marked and redone by a warp with buffers for all
+// 100.  Every sum keeps the reference's order.  All arithmetic uses
+// explicitly rounded operations (no fused multiply-add), so the float
+// results agree with the reference's x86-64 build bit for bit; exp, pow and
+// log are CUDA's double-precision functions.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -81,8 +81,11 @@ __device__ long gcd_long(long a, long b) {
   return a;
 }
 
+// (sp[i * kStride]: the probability of score i)
+
 // sum_i sp[i] exp(x i) the way the reference forms it: a running power
 // from pow(exp(x), lo - 1), or exp(x i) per term once that underflows
+template <int kStride>
 __device__ double power_sum(const double *sp, int lo, int hi, double x) {
   const double x0 = exp(x);
   double x1 = pow(x0, (double)(lo - 1));
@@ -90,26 +93,27 @@ __device__ double power_sum(const double *sp, int lo, int hi, double x) {
   if (x1 > 0.0) {
     for (int i = lo; i <= hi; ++i) {
       x1 = dmul(x1, x0);
-      sum = dadd(sum, dmul(sp[i], x1));
+      sum = dadd(sum, dmul(sp[i * kStride], x1));
     }
   } else {
-    for (int i = lo; i <= hi; ++i) sum = dadd(sum, dmul(sp[i], exp(dmul(x, (double)i))));
+    for (int i = lo; i <= hi; ++i) sum = dadd(sum, dmul(sp[i * kStride], exp(dmul(x, (double)i))));
   }
   return sum;
 }
 
 // lambda by bisection (BlastKarlinLambdaBis)
+template <int kStride>
 __device__ double lambda_bisect(const double *sp, int lo, int hi) {
   if (range_bad(lo, hi)) return -1.0;
   double lambda = 0.0, up = 0.5;
   for (int guard = 0; guard < 2048; ++guard) {
     up = dmul(up, 2.0);
-    if (power_sum(sp, lo, hi, up) >= 1.0) break;
+    if (power_sum<kStride>(sp, lo, hi, up) >= 1.0) break;
     lambda = up;
   }
   for (int j = 0; j < 17; ++j) {
     const double mid = ddiv(dadd(lambda, up), 2.0);
-    if (power_sum(sp, lo, hi, mid) > 1.0)
+    if (power_sum<kStride>(sp, lo, hi, mid) > 1.0)
       up = mid;
     else
       lambda = mid;
@@ -118,6 +122,7 @@ __device__ double lambda_bisect(const double *sp, int lo, int hi) {
 }
 
 // lambda by Newton-Raphson from 0.5 (BlastKarlinLambdaNR)
+template <int kStride>
 __device__ double lambda_newton(const double *sp, int lo, int hi) {
   if (range_bad(lo, hi)) return -1.0;
   double lambda = 0.5;
@@ -129,7 +134,7 @@ __device__ double lambda_newton(const double *sp, int lo, int hi) {
     if (x1 == 0.0) break;
     for (int i = lo; i <= hi; ++i) {
       x1 = dmul(x1, x0);
-      const double t = dmul(sp[i], x1);
+      const double t = dmul(sp[i * kStride], x1);
       sum = dadd(sum, t);
       slope = dadd(slope, dmul(t, (double)i));
     }
@@ -140,10 +145,11 @@ __device__ double lambda_newton(const double *sp, int lo, int hi) {
       break;
     }
   }
-  return lambda_bisect(sp, lo, hi);
+  return lambda_bisect<kStride>(sp, lo, hi);
 }
 
 // relative entropy (BlastKarlinLtoH)
+template <int kStride>
 __device__ double entropy(const double *sp, int lo, int hi, double lambda) {
   if (lambda < 0.0 || range_bad(lo, hi)) return -1.0;
   const double etolam = exp(lambda);
@@ -151,14 +157,231 @@ __device__ double entropy(const double *sp, int lo, int hi, double lambda) {
   if (etolami > 0.0) {
     for (int s = lo; s <= hi; ++s) {
       etolami = dmul(etolami, etolam);
-      av = dadd(av, dmul(dmul(sp[s], (double)s), etolami));
+      av = dadd(av, dmul(dmul(sp[s * kStride], (double)s), etolami));
     }
   } else {
     for (int s = lo; s <= hi; ++s)
-      av = dadd(av, dmul(dmul(sp[s], (double)s), exp(dmul(lambda, (double)s))));
+      av = dadd(av, dmul(dmul(sp[s * kStride], (double)s), exp(dmul(lambda, (double)s))));
   }
   return dmul(lambda, av);
 }
+
+// K from the series' state after its rounds (sum: the last term; p[i *
+// stride]: probability of score low + i); -1 where it has no value
+__device__ double karlin_k(double sum, double oldsum, double oldsum2, double Sum, int j,
+                           double av, double etolam, double lambda, int low, int range,
+                           const double *p, int stride) {
+  double sumlimit = 0.01;
+  const double ratio = ddiv(oldsum, oldsum2);
+  if (ratio >= dsub(1.0, dmul(sumlimit, 0.001))) return -1.0;
+  sumlimit = dmul(sumlimit, 0.01);
+  while (sum > sumlimit) {
+    oldsum = dmul(oldsum, ratio);
+    ++j;
+    sum = ddiv(oldsum, (double)j);
+    Sum = dadd(Sum, sum);
+  }
+  long delta = -low;
+  for (int i = 1; i <= range && delta > 1; ++i)
+    if (p[i * stride] != 0.0) delta = gcd_long(delta, i);
+  const double e2 = exp(dmul(-2.0, Sum));
+  if (dmul((double)delta, etolam) > 0.05) {
+    const double etolami = pow(etolam, (double)(-delta));
+    return ddiv(dmul((double)delta, e2), dmul(av, dsub(1.0, etolami)));
+  }
+  return ddiv(dmul((double)(-delta), e2),
+              dmul(av, dsub(exp(dmul((double)(-delta), lambda)), 1.0)));
+}
+
+// NormalizedCutoff2NominalCutoff and Normalized2Nominal in float; ln K is
+// the float nearest the exact logarithm
+__device__ void store_cutoffs(const KarlinArgs &a, uint32_t r, float l, float h, double K,
+                              int32_t *cutoffs, int32_t *triggers, float *karlin) {
+  const float k = (float)K;
+  const float c = __fdiv_rn(__fmul_rn(a.ungapped_bits, a.ln2), l);
+  const float t =
+      __fdiv_rn(__fadd_rn(__fmul_rn(a.trigger_bits, a.ln2), (float)log((double)k)), l);
+  cutoffs[r] = (int32_t)floorf(c);
+  triggers[r] = (int32_t)floorf(t);
+  if (karlin) {
+    karlin[3 * (size_t)r] = l;
+    karlin[3 * (size_t)r + 1] = k;
+    karlin[3 * (size_t)r + 2] = h;
+  }
+}
+
+// kGroup lanes a query, 32 / kGroup queries a block (of one warp).  A query's
+// convolutions are some 25,000 multiplications and additions, and each of
+// its serial sums would keep only one lane of a warp busy, so with many
+// queries those go side by side.  One buffer a query, in shared memory, its
+// entries a row apart: a round replaces it from its end, kOut entries a lane
+// at a time, each of which reads only entries up to its own.  The entries
+// slide through registers: a step is a load of an entry and one of a
+// probability for kOut products, and rows of zeros below and above the
+// entries take the place of bounds (a zero's term leaves a sum as it is).
+// What bounds it is the latency of double precision chains: the shared memory
+// holds the buffers of some 88 queries an SM, which four lanes a query make
+// eleven warps.  150,000 reads' frames: 4.61 ms with a warp a query, 2.43 with
+// a lane, 1.58 with two, 1.41 with four.  `rounds`: those the buffer holds
+// (karlin_rounds).
+constexpr int kOut = 8;
+constexpr int kGroup = 4;
+constexpr int kRow = 32 / kGroup;  // queries a block: entries of a row
+
+__host__ __device__ constexpr int karlin_steps(int range) {  // scores, a multiple of kOut
+  return (range + kOut) / kOut * kOut;
+}
+
+__global__ void __launch_bounds__(32)
+    karlin_group_kernel(KarlinArgs a, const uint8_t *__restrict__ codes,
+                        const uint64_t *__restrict__ offsets,
+                        const uint32_t *__restrict__ lengths, uint32_t n, int rounds,
+                        int32_t *__restrict__ cutoffs, int32_t *__restrict__ triggers,
+                        float *__restrict__ karlin) {
+  extern __shared__ double columns[];
+  const int lane = threadIdx.x, column = lane % kRow, part = lane / kRow;
+  const int low = a.low, high = a.high, range = high - low;
+  const int steps = karlin_steps(range);
+  double *p = columns + column;          // [steps]: zero past the range
+  double *buf = p + kRow * 2 * steps;    // [-steps ..]: zero rows below the entries
+  const int rows = rounds * range + 1 + kOut * kGroup;
+  const uint32_t r0 = blockIdx.x * kRow, r = r0 + column;
+  const int nl = a.number_letters;
+  // compositions (the warp counts one query after the other), then
+  // frequencies with a pseudo-count for absent letters, normalised
+  int *count = reinterpret_cast<int *>(columns + kRow * (2 * steps + kMaxLetters));
+  for (int i = lane; i < 33 * kRow; i += 32) count[i] = 0;
+  const uint64_t offset = r < n ? offsets[r] : 0;
+  const uint32_t length = r < n ? lengths[r] : 0;
+  __syncwarp();
+  for (int k = 0; k < kRow && r0 + k < n; ++k) {
+    const uint8_t *q = codes + __shfl_sync(0xffffffffu, offset, k);
+    const uint32_t len = __shfl_sync(0xffffffffu, length, k);
+#pragma unroll 4
+    for (uint32_t i = lane; i < len; i += 32) {
+      const uint8_t c = q[i];
+      if (c <= kMaxRegular) atomicAdd(&count[33 * k + c], 1);
+    }
+  }
+  __syncwarp();
+  double total = 0.0;
+  for (int c = 0; c < nl; ++c) {
+    const int k = count[33 * column + c];
+    const double f = (double)k + (k < 1 ? 1.0 : 0.0);
+    buf[kRow * c] = f;
+    total = dadd(total, f);
+  }
+  __syncwarp();
+  for (int c = part; c < nl; c += kGroup) buf[kRow * c] = ddiv(buf[kRow * c], total);
+  __syncwarp();
+  double s = 0.0;
+  for (int i = 0; i <= range; ++i) {
+    double acc = 0.0;
+    for (int k = a.pair_begin[i]; k < a.pair_begin[i + 1]; ++k)
+      acc = dadd(acc, dmul(buf[kRow * a.pair_c1[k]], a.background[a.pair_c2[k]]));
+    p[kRow * i] = acc;
+    if (acc > 0.0) s = dadd(s, acc);
+  }
+  __syncwarp();
+  for (int i = part; i < steps; i += kGroup)
+    p[kRow * i] = i <= range ? (p[kRow * i] > 0.0 ? ddiv(p[kRow * i], s) : p[kRow * i]) : 0.0;
+  for (int i = part - steps; i < rows; i += kGroup) buf[kRow * i] = i == 0 ? 1.0 : 0.0;
+  __syncwarp();
+  const double *sp = p - kRow * low;
+  const float l = (float)lambda_newton<kRow>(sp, low, high);
+  const float h = (float)entropy<kRow>(sp, low, high, (double)l);
+  const double lambda = (double)l, H = (double)h;
+  const double av = ddiv(H, lambda), etolam = exp(lambda);
+  const bool valid = r < n && lambda > 0.0 && H > 0.0, closed = low == -1 || high == 1;
+  double sum = 1.0, oldsum = 1.0, oldsum2 = 1.0, Sum = 0.0;
+  int j = 0;
+  // (every lane takes part in the rounds, for the queries still in need)
+  bool open = valid && !closed;
+  for (int round = 0; round < rounds && __any_sync(0xffffffffu, open); ++round) {
+    const int top = (round + 1) * range;  // the last entry after this round
+    for (int k0 = top / (kOut * kGroup) * (kOut * kGroup); k0 >= 0; k0 -= kOut * kGroup) {
+      double *at = buf + kRow * (k0 + kOut * part);
+      double acc[kOut], w[kOut], next[kOut];
+#pragma unroll
+      for (int e = 0; e < kOut; ++e) {
+        acc[e] = 0.0;
+        w[e] = at[kRow * e];
+      }
+      for (int u0 = 0; u0 < steps; u0 += kOut) {
+#pragma unroll
+        for (int e = 0; e < kOut; ++e) next[e] = at[-kRow * (u0 + 1 + e)];
+#pragma unroll
+        for (int t = 0; t < kOut; ++t) {
+          const double pu = p[kRow * (u0 + t)];
+#pragma unroll
+          for (int e = 0; e < kOut; ++e)
+            acc[e] = dadd(acc[e], dmul(e >= t ? w[e - t] : next[t - e - 1], pu));
+        }
+#pragma unroll
+        for (int e = 0; e < kOut; ++e) w[e] = next[kOut - 1 - e];
+      }
+      __syncwarp();
+#pragma unroll
+      for (int e = 0; e < kOut; ++e) at[kRow * e] = acc[e];
+      __syncwarp();
+    }
+    if (open) {
+      const int lo = (round + 1) * low;
+      double etolami = pow(etolam, (double)(lo - 1));
+      s = 0.0;
+      int i = 0;
+#pragma unroll 4
+      for (; i < -lo; ++i) {
+        etolami = dmul(etolami, etolam);
+        s = dadd(s, dmul(buf[kRow * i], etolami));
+      }
+#pragma unroll 4
+      for (; i <= top; ++i) s = dadd(s, buf[kRow * i]);
+      oldsum2 = oldsum;
+      oldsum = s;
+      ++j;
+      sum = ddiv(s, (double)j);
+      Sum = dadd(Sum, sum);
+      open = sum > 0.01;
+    }
+    __syncwarp();
+  }
+  if (r >= n || part != 0) return;
+  if (open) {
+    cutoffs[r] = kPending;
+    return;
+  }
+  double K = -1.0;
+  if (valid)
+    K = closed ? dmul(av, dsub(1.0, ddiv(1.0, etolam)))
+               : karlin_k(sum, oldsum, oldsum2, Sum, j, av, etolam, lambda, low, range, p, kRow);
+  store_cutoffs(a, r, l, h, K, cutoffs, triggers, karlin);
+}
+
+// Rounds karlin_group_kernel's buffers hold, so that eleven blocks share an
+// SM's 228 KB (and 24 at most: the series ends after 12 to 15 rounds for
+// nearly every composition); their bytes.
+int karlin_rounds(int range, size_t *bytes) {
+  const size_t most = 20172, row = kRow * sizeof(double);
+  const int steps = karlin_steps(range), extra = 2 * steps + kOut * kGroup + 1;
+  int rounds = ((int)(most / row) - extra) / range;
+  if (rounds > kFastIter) rounds = kFastIter;
+  if (rounds < 1) rounds = 1;
+  int rows = extra + rounds * range;
+  // (the compositions' counts lie above the frequencies)
+  const int start = 2 * steps + kMaxLetters + (int)((33 * kRow * sizeof(int) + row - 1) / row);
+  if (rows < start) rows = start;
+  *bytes = rows * row;
+  return rounds;
+}
+
+// From this many queries on, karlin_group_kernel is the faster: 103 us from 1
+// to 3,000 queries of 308 residues and 133 us of 2,000, where a warp a query
+// takes 94 and 96 at 1,500, 109 and 111 at 2,000, 144 and 147 at 3,000.
+constexpr uint32_t kGroupQueries = 2048;
+// And where its buffers hold the rounds that most queries need (a range of up
+// to 15 scores; a wider one takes a warp a query).
+constexpr int kGroupRounds = 15;
 
 // kIter: rounds of the K series the buffers hold.  kRetry: the second pass
 // (only queries whose cutoff holds kPending).  The first pass runs eight
@@ -180,8 +403,21 @@ __global__ void __launch_bounds__(kWarps * 32, kRetry ? 1 : 8)
   double *buf0 = dist + (size_t)w * 2 * cap, *buf1 = buf0 + cap;
   const int nl = a.number_letters;
   const uint32_t warps = gridDim.x * kWarps;
-  for (uint32_t r = blockIdx.x * kWarps + w; r < n; r += warps) {
-    if (kRetry && cutoffs[r] != kPending) continue;
+  uint32_t first = 0, marked = 0;  // marked ones of the 32 queries from `first` on (kRetry)
+  for (uint64_t at = (uint64_t)(blockIdx.x * kWarps + w) * (kRetry ? 32 : 1); at < n || marked;) {
+    uint32_t r = (uint32_t)at;
+    if (kRetry) {
+      if (!marked) {
+        first = (uint32_t)at;
+        marked = __ballot_sync(0xffffffffu, at + lane < n && cutoffs[at + lane] == kPending);
+        at += 32ull * warps;
+        if (!marked) continue;
+      }
+      r = first + __ffs(marked) - 1;
+      marked &= marked - 1;
+    } else {
+      at += warps;
+    }
     // composition of regular letters over the whole query
     count[w][lane] = 0;
     __syncwarp();
@@ -223,8 +459,8 @@ __global__ void __launch_bounds__(kWarps * 32, kRetry ? 1 : 8)
     // lambda and H on lane 0, rounded to float as BlastKarlinBlkCalc keeps them
     float l = 0.f, h = 0.f;
     if (lane == 0) {
-      l = (float)lambda_newton(sp, low, high);
-      h = (float)entropy(sp, low, high, (double)l);
+      l = (float)lambda_newton<1>(sp, low, high);
+      h = (float)entropy<1>(sp, low, high, (double)l);
     }
     l = __shfl_sync(0xffffffffu, l, 0);
     h = __shfl_sync(0xffffffffu, h, 0);
@@ -277,47 +513,14 @@ __global__ void __launch_bounds__(kWarps * 32, kRetry ? 1 : 8)
           sum = ddiv(s, (double)j);
           Sum = dadd(Sum, sum);
         }
-        const double ratio = ddiv(oldsum, oldsum2);
-        if (kIter < kKarlinIterMax && j == kIter && sum > sumlimit) {
+        if (kIter < kKarlinIterMax && j == kIter && sum > sumlimit)
           pending = true;
-        } else if (!(ratio >= dsub(1.0, dmul(sumlimit, 0.001)))) {
-          sumlimit = dmul(sumlimit, 0.01);
-          while (sum > sumlimit) {
-            oldsum = dmul(oldsum, ratio);
-            ++j;
-            sum = ddiv(oldsum, (double)j);
-            Sum = dadd(Sum, sum);
-          }
-          long delta = -low;
-          for (int i = 1; i <= range && delta > 1; ++i)
-            if (p[i] != 0.0) delta = gcd_long(delta, i);
-          const double e2 = exp(dmul(-2.0, Sum));
-          if (dmul((double)delta, etolam) > 0.05) {
-            const double etolami = pow(etolam, (double)(-delta));
-            K = ddiv(dmul((double)delta, e2), dmul(av, dsub(1.0, etolami)));
-          } else {
-            K = ddiv(dmul((double)(-delta), e2),
-                     dmul(av, dsub(exp(dmul((double)(-delta), lambda)), 1.0)));
-          }
-        }
+        else
+          K = karlin_k(sum, oldsum, oldsum2, Sum, j, av, etolam, lambda, low, range, p, 1);
       }
     }
     if (lane == 0 && pending) cutoffs[r] = kPending;
-    if (lane == 0 && !pending) {
-      const float k = (float)K;
-      // NormalizedCutoff2NominalCutoff and Normalized2Nominal in float; ln K
-      // is the float nearest the exact logarithm
-      const float c = __fdiv_rn(__fmul_rn(a.ungapped_bits, a.ln2), l);
-      const float t =
-          __fdiv_rn(__fadd_rn(__fmul_rn(a.trigger_bits, a.ln2), (float)log((double)k)), l);
-      cutoffs[r] = (int32_t)floorf(c);
-      triggers[r] = (int32_t)floorf(t);
-      if (karlin) {
-        karlin[3 * (size_t)r] = l;
-        karlin[3 * (size_t)r + 1] = k;
-        karlin[3 * (size_t)r + 2] = h;
-      }
-    }
+    if (lane == 0 && !pending) store_cutoffs(a, r, l, h, K, cutoffs, triggers, karlin);
     __syncwarp();
   }
 }
@@ -384,13 +587,24 @@ extern "C" int gzb_query_karlin_cutoffs(const uint8_t *d_codes, const uint64_t *
   auto full = karlin_kernel<kFullWarps, kKarlinIterMax, true>;
   GZB_CUDA(cudaFuncSetAttribute(fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fast));
   GZB_CUDA(cudaFuncSetAttribute(full, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_full));
-  const uint64_t want_fast = (number_queries + kFastWarps - 1) / kFastWarps;
-  const uint64_t most_fast = (uint64_t)sms * 8;
-  fast<<<(unsigned)(want_fast < most_fast ? want_fast : most_fast), kFastWarps * 32, smem_fast,
-         (cudaStream_t)stream>>>(a, d_codes, d_offsets, d_lengths, number_queries, d_cutoffs,
-                                 d_triggers, d_karlin);
+  size_t smem_group = 0;
+  const int rounds = karlin_rounds(range, &smem_group);
+  if (number_queries >= kGroupQueries && rounds >= kGroupRounds) {
+    GZB_CUDA(cudaFuncSetAttribute(karlin_group_kernel,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_group));
+    karlin_group_kernel<<<(number_queries + kRow - 1) / kRow, 32, smem_group,
+                          (cudaStream_t)stream>>>(
+        a, d_codes, d_offsets, d_lengths, number_queries, rounds, d_cutoffs, d_triggers,
+        d_karlin);
+  } else {
+    const uint64_t want_fast = (number_queries + kFastWarps - 1) / kFastWarps;
+    const uint64_t most_fast = (uint64_t)sms * 8;
+    fast<<<(unsigned)(want_fast < most_fast ? want_fast : most_fast), kFastWarps * 32, smem_fast,
+           (cudaStream_t)stream>>>(a, d_codes, d_offsets, d_lengths, number_queries, d_cutoffs,
+                                   d_triggers, d_karlin);
+  }
   GZB_CUDA(cudaGetLastError());
-  const uint64_t want_full = (number_queries + kFullWarps - 1) / kFullWarps;
+  const uint64_t want_full = (number_queries + 32 * kFullWarps - 1) / (32 * kFullWarps);
   const uint64_t most_full = (uint64_t)sms * 4;
   full<<<(unsigned)(want_full < most_full ? want_full : most_full), kFullWarps * 32, smem_full,
          (cudaStream_t)stream>>>(a, d_codes, d_offsets, d_lengths, number_queries, d_cutoffs,
