@@ -76,6 +76,69 @@ __device__ __forceinline__ int seg_class(uint8_t v) {
   return c < 20 ? c : -1;
 }
 
+// The entropy tables in shared memory: lanes look different entries up,
+// which the parameter bank answers one at a time.
+struct SegTables {
+  double entropy12[kSegWindow + 1];
+  double log_ratio[kSegWindow][kSegWindow + 1];
+};
+
+__device__ __forceinline__ void load_seg_tables(const SegArgs &a, SegTables &t) {
+  for (int i = threadIdx.x; i <= kSegWindow; i += blockDim.x) t.entropy12[i] = a.entropy12[i];
+  for (int i = threadIdx.x; i < kSegWindow * (kSegWindow + 1); i += blockDim.x)
+    t.log_ratio[i / (kSegWindow + 1)][i % (kSegWindow + 1)] =
+        a.log_ratio[i / (kSegWindow + 1)][i % (kSegWindow + 1)];
+  __syncthreads();
+}
+
+// A window's composition in registers (arrays with a letter's index would
+// be local memory): a 4-bit count a letter, and how many letters occur v
+// times, 5 bits a value v.  On the frames of 150,000 reads of 150 bases the
+// scan took 0.76 ms with byte arrays and takes 0.47; the search, whose
+// windows and trimmed stretches were sorted in arrays and whose positions
+// every lane walked, 2.96 and 1.06.
+struct SegWindowCounts {
+  uint32_t count[3] = {0, 0, 0};
+  uint64_t per = 20;
+  int total = 0;
+
+  __device__ __forceinline__ int of(int k) const {
+    return ((k < 8 ? count[0] : k < 16 ? count[1] : count[2]) >> (4 * (k & 7))) & 15;
+  }
+  __device__ __forceinline__ void add(int k) {
+    const int c = of(k);
+    const uint32_t one = 1u << (4 * (k & 7));
+    count[0] += k < 8 ? one : 0;
+    count[1] += k >= 8 && k < 16 ? one : 0;
+    count[2] += k >= 16 ? one : 0;
+    per += (32ull << (5 * c)) - (1ull << (5 * c));
+    ++total;
+  }
+  __device__ __forceinline__ void remove(int k) {
+    const int c = of(k);
+    const uint32_t one = 1u << (4 * (k & 7));
+    count[0] -= k < 8 ? one : 0;
+    count[1] -= k >= 8 && k < 16 ? one : 0;
+    count[2] -= k >= 16 ? one : 0;
+    per -= (1ull << (5 * c)) - (1ull << (5 * (c - 1)));
+    --total;
+  }
+  // seg_entropy of the counts: the same sums, the largest counts first
+  __device__ __forceinline__ double entropy(const SegTables &t, double ln2) const {
+    const double *term = total == kSegWindow ? t.entropy12 : t.log_ratio[total];
+    double ent = 0.0;
+    for (uint64_t x = per & ~31ull; x != 0;) {
+      const int v = (63 - __clzll((long long)x)) / 5;
+      const double w =
+          total == kSegWindow ? term[v] : __dmul_rn((double)v, term[v]);
+      for (int n = (int)(x >> (5 * v)); n > 0; --n) ent = __dadd_rn(ent, w);
+      x &= (1ull << (5 * v)) - 1;
+    }
+    if (total == kSegWindow || total == 0) return ent;
+    return __ddiv_rn(__dmul_rn(-ent, __ddiv_rn(1.0, (double)total)), ln2);
+  }
+};
+
 // counts of the letters in s[0..n), decreasing, 0-terminated
 __device__ void seg_state(const uint8_t *s, int n, int *comp, int *state) {
   for (int k = 0; k < 20; ++k) comp[k] = 0;
@@ -163,6 +226,67 @@ __device__ double seg_probability(const SegArgs &a, const int *state, int total)
   return __dsub_rn(__dadd_rn(ass, perm), __dmul_rn((double)total, a.ln20));
 }
 
+// seg_state and seg_probability of a stretch of at most 127 letters in
+// registers, a byte a letter's count and a byte a sorted count.
+struct SegSorted {
+  uint32_t count[5] = {0, 0, 0, 0, 0}, state[5] = {0, 0, 0, 0, 0};
+
+  // adds `d` to letter k's count, which becomes `c`, and to the sorted count
+  // of rank `at`
+  __device__ __forceinline__ void change(int k, int at, uint32_t d) {
+#pragma unroll
+    for (int w = 0; w < 5; ++w) {
+      count[w] += w == (k >> 2) ? d << (8 * (k & 3)) : 0;
+      state[w] += w == (at >> 2) ? d << (8 * (at & 3)) : 0;
+    }
+  }
+  __device__ __forceinline__ int of(int k) const {
+    const int w = k >> 2;
+    const uint32_t x = w == 0 ? count[0] : w == 1 ? count[1] : w == 2 ? count[2]
+                       : w == 3 ? count[3] : count[4];
+    return (x >> (8 * (k & 3))) & 255;
+  }
+  // sorted counts of at least c (1 <= c <= 128)
+  __device__ __forceinline__ int at_least(int c) const {
+    uint32_t m = 0;
+#pragma unroll
+    for (int w = 0; w < 5; ++w)
+      m |= (((state[w] | 0x80808080u) - (uint32_t)c * 0x01010101u) & 0x80808080u) >> w;
+    return __popc(m);
+  }
+  // the first sorted count equal to the letter's grows, the last one shrinks
+  __device__ __forceinline__ void add(int k) { change(k, at_least(of(k) + 1), 1u); }
+  __device__ __forceinline__ void remove(int k) {
+    change(k, at_least(of(k)) - 1, 0xffffffffu);
+  }
+  __device__ __forceinline__ double probability(const SegArgs &a, int total) const {
+    const double *T = g_seg_ln_fact;
+    double ass = T[20], perm = T[total];
+    int run = 0, prev = (int)(state[0] & 255u);
+    if (prev != 0) {
+#pragma unroll
+      for (int i = 0; i < 20; ++i) {
+        const int v = (state[i / 4] >> (8 * (i & 3))) & 255;
+        if (v != prev) {
+          ass = __dsub_rn(ass, T[run]);
+          run = 0;
+          if (v == 0) {
+            run = 20 - i;
+            break;
+          }
+        }
+        perm = __dsub_rn(perm, T[v]);
+        ++run;
+        prev = v;
+      }
+      ass = __dsub_rn(ass, T[run]);
+    }
+    return __dsub_rn(__dadd_rn(ass, perm), __dmul_rn((double)total, a.ln20));
+  }
+};
+
+constexpr int kSegSorted = 127;  // letters whose counts fit SegSorted
+
 // The least probable sub-window of s[0..n) over lengths n .. max(1, n-100)+1
 // (the reference's first minimum in the order length descending, start
 // ascending).  The whole warp calls it with the same arguments: lane l
@@ -175,8 +299,29 @@ __device__ void seg_trim_warp(const SegArgs &a, const uint8_t *s, int n, int *le
   const int lens = n - min_length;  // lengths n, n-1, ..., min_length+1
   double best = 1.0;
   uint64_t best_at = ~0ull;         // (length rank, start)
+  if (n <= kSegSorted) {
+    for (int li = lane; li < lens; li += 32) {
+      const int len = n - li;
+      SegSorted sorted;
+      for (int i = 0; i < len; ++i) {
+        const int k = seg_class(s[i]);
+        if (k >= 0) sorted.add(k);
+      }
+      for (int i = 0;; ++i) {
+        const double p = sorted.probability(a, len);
+        if (p < best) {
+          best = p;
+          best_at = ((uint64_t)li << 32) | (uint32_t)i;
+        }
+        if (i + 1 + len > n) break;
+        const int out = seg_class(s[i]), in = seg_class(s[i + len]);
+        if (out >= 0) sorted.remove(out);
+        if (in >= 0) sorted.add(in);
+      }
+    }
+  }
   int comp[20], state[21];
-  for (int li = lane; li < lens; li += 32) {
+  for (int li = lane; li < lens && n > kSegSorted; li += 32) {
     const int len = n - li;
     seg_state(s, len, comp, state);
     for (int i = 0;; ++i) {
@@ -221,8 +366,7 @@ struct SegFrame {
 
 // Masks the low-complexity segments of s[0..n) (n >= the window); every
 // lane of the warp runs the same search on the same data (so its branches
-// agree), the trimming is split over the lanes, and lane 0 writes the
-// masks.  E, when given, holds the entropy of the window starting at every
+// agree), the trimming and the masks are split over the lanes.  E, when given, holds the entropy of the window starting at every
 // position 0 .. n-12 of s (computed before any mask), so the search reads
 // H instead of computing it; a frame's H(i) is that of the window starting
 // at its position min(i, its length - 12).  Returns false if the search
@@ -256,19 +400,45 @@ __device__ bool seg_sequence(const SegArgs &a, uint8_t *s, int n, int lane, cons
         }
         ++start;
       }
-      if ((E ? h_at(i) : seg_entropy(a, state)) > kSegLowCut) continue;
-      int lo = i;
-      while (lo >= f.left_limit && (E ? h_at(lo) : seg_h(a, w, f.n, lo)) <= kSegHighCut) --lo;
-      const int left_i = lo + 1;
-      int hi = i;
-      while (hi <= f.n - 1 && (E ? h_at(hi) : seg_h(a, w, f.n, hi)) <= kSegHighCut) ++hi;
-      const int right_i = hi - 1;
+      if (E) {  // 32 positions at a time
+        unsigned low;
+        for (;; i += 32) {
+          low = __ballot_sync(0xffffffffu, i + lane < f.n && h_at(i + lane) <= kSegLowCut);
+          if (low || i + 32 >= f.n) break;
+        }
+        if (!low) break;
+        i += __ffs(low) - 1;
+      } else if (seg_entropy(a, state) > kSegLowCut) {
+        continue;
+      }
+      int lo = i, hi = i;
+      if (E) {
+        for (unsigned stop = 0;; lo -= 32) {
+          stop = __ballot_sync(0xffffffffu, lo - lane < f.left_limit ||
+                                                !(h_at(lo - lane) <= kSegHighCut));
+          if (stop) {
+            lo -= __ffs(stop) - 1;
+            break;
+          }
+        }
+        for (unsigned stop = 0;; hi += 32) {
+          stop = __ballot_sync(0xffffffffu, hi + lane > f.n - 1 ||
+                                                !(h_at(hi + lane) <= kSegHighCut));
+          if (stop) {
+            hi += __ffs(stop) - 1;
+            break;
+          }
+        }
+      } else {
+        while (lo >= f.left_limit && seg_h(a, w, f.n, lo) <= kSegHighCut) --lo;
+        while (hi <= f.n - 1 && seg_h(a, w, f.n, hi) <= kSegHighCut) ++hi;
+      }
+      const int left_i = lo + 1, right_i = hi - 1;
       int left_end = left_i, right_end = right_i;
       seg_trim_warp(a, w + left_end, right_end - left_end + 1, &left_end, &right_end, lane);
       // the mask bit is invisible to seg_class, so the other lanes' reads
       // see the same letters whichever value they load
-      if (lane == 0)
-        for (int k = left_end; k <= right_end; ++k) s[f.base + k] |= kMaskBit;
+      for (int k = left_end + lane; k <= right_end; k += 32) s[f.base + k] |= kMaskBit;
       const int next = right_i < right_end ? right_i : right_end;
       const bool child = i < left_end && left_end - left_i >= kSegWindow;
       // the frame resumes after the segment
@@ -331,6 +501,8 @@ __global__ void __launch_bounds__(kSegBlock)
     seg_scan_kernel(SegArgs a, uint8_t *__restrict__ codes, const uint64_t *__restrict__ offsets,
                     const uint32_t *__restrict__ lengths, uint64_t units, int mode,
                     uint32_t *__restrict__ status) {
+  __shared__ SegTables tables;
+  load_seg_tables(a, tables);
   for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < units;
        u += (uint64_t)gridDim.x * blockDim.x) {
     int n;
@@ -346,52 +518,23 @@ __global__ void __launch_bounds__(kSegBlock)
       for (int i = 0; i < n; ++i) s[i] = finish_code(s[i]);
       continue;
     }
-    uint8_t comp[20];
-    uint8_t per[kSegWindow + 1];  // per[v]: letters occurring v times
-    for (int k = 0; k < 20; ++k) comp[k] = 0;
-    for (int v = 0; v <= kSegWindow; ++v) per[v] = 0;
-    int total = 0;
+    SegWindowCounts counts;
     bool marked = false, shifted = false;
     for (int i = 0; i < kSegWindow; ++i) {
       const int k = seg_class(s[i]);
       shifted |= (s[i] & 63) >= 32;
-      if (k >= 0) {
-        ++comp[k];
-        ++total;
-      }
+      if (k >= 0) counts.add(k);
     }
-    for (int k = 0; k < 20; ++k) ++per[comp[k]];
     for (int start = 0;; ++start) {
-      double ent = 0.0;
-      if (total == kSegWindow) {
-        for (int v = kSegWindow; v >= 1; --v)
-          for (int t = 0; t < per[v]; ++t) ent = __dadd_rn(ent, a.entropy12[v]);
-      } else if (total > 0) {
-        const double r = __ddiv_rn(1.0, (double)total);
-        for (int v = total; v >= 1; --v)
-          for (int t = 0; t < per[v]; ++t)
-            ent = __dadd_rn(ent, __dmul_rn((double)v, a.log_ratio[total][v]));
-        ent = __ddiv_rn(__dmul_rn(-ent, r), a.ln2);
-      }
-      if (ent <= kSegLowCut) {
+      if (counts.entropy(tables, a.ln2) <= kSegLowCut) {
         marked = true;
         break;
       }
       if (start + kSegWindow >= n) break;
       const int out = seg_class(s[start]), in = seg_class(s[start + kSegWindow]);
       shifted |= (s[start + kSegWindow] & 63) >= 32;
-      if (out >= 0) {
-        --per[comp[out]];
-        --comp[out];
-        ++per[comp[out]];
-        --total;
-      }
-      if (in >= 0) {
-        --per[comp[in]];
-        ++comp[in];
-        ++per[comp[in]];
-        ++total;
-      }
+      if (out >= 0) counts.remove(out);
+      if (in >= 0) counts.add(in);
     }
     if (marked) {
       s[0] |= 128;
@@ -411,6 +554,8 @@ __global__ void __launch_bounds__(kSegBlock)
                          const uint64_t *__restrict__ offsets,
                          const uint32_t *__restrict__ lengths, uint64_t units, int mode,
                          uint32_t *__restrict__ status) {
+  __shared__ SegTables tables;
+  load_seg_tables(a, tables);
   const int lane = threadIdx.x & 31;
   const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t u = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; u < units;
@@ -434,49 +579,20 @@ __global__ void __launch_bounds__(kSegBlock)
     const int run = (m + 31) / 32, p0 = lane * run, p1 = min(p0 + run, m);
     bool low = false;
     if (p0 < p1) {
-      uint8_t comp[20];
-      uint8_t per[kSegWindow + 1];  // per[v]: letters occurring v times
-      for (int k = 0; k < 20; ++k) comp[k] = 0;
-      for (int v = 0; v <= kSegWindow; ++v) per[v] = 0;
-      int total = 0;
+      SegWindowCounts counts;
       for (int i = p0; i < p0 + kSegWindow; ++i) {
         const int k = seg_class(s[i]);
-        if (k >= 0) {
-          ++comp[k];
-          ++total;
-        }
+        if (k >= 0) counts.add(k);
       }
-      for (int k = 0; k < 20; ++k) ++per[comp[k]];
       for (int start = p0;; ++start) {
-        double ent = 0.0;
-        if (total == kSegWindow) {
-          for (int v = kSegWindow; v >= 1; --v)
-            for (int t = 0; t < per[v]; ++t) ent = __dadd_rn(ent, a.entropy12[v]);
-        } else if (total > 0) {
-          const double r = __ddiv_rn(1.0, (double)total);
-          for (int v = total; v >= 1; --v)
-            for (int t = 0; t < per[v]; ++t)
-              ent = __dadd_rn(ent, __dmul_rn((double)v, a.log_ratio[total][v]));
-          ent = __ddiv_rn(__dmul_rn(-ent, r), a.ln2);
-        }
-        if (ent <= kSegLowCut) {
+        if (counts.entropy(tables, a.ln2) <= kSegLowCut) {
           low = true;
           break;
         }
         if (start + 1 >= p1) break;
         const int out = seg_class(s[start]), in = seg_class(s[start + kSegWindow]);
-        if (out >= 0) {
-          --per[comp[out]];
-          --comp[out];
-          ++per[comp[out]];
-          --total;
-        }
-        if (in >= 0) {
-          --per[comp[in]];
-          ++comp[in];
-          ++per[comp[in]];
-          ++total;
-        }
+        if (out >= 0) counts.remove(out);
+        if (in >= 0) counts.add(in);
       }
     }
     const bool marked = __any_sync(0xffffffffu, low);
@@ -496,16 +612,33 @@ __global__ void __launch_bounds__(kSegBlock)
                       const uint32_t *__restrict__ lengths, uint64_t units, int mode,
                       uint32_t *__restrict__ status, int cache) {
   extern __shared__ double ecache[];  // [warps of the block][cache]
+  __shared__ SegTables tables;
+  load_seg_tables(a, tables);
   const int lane = threadIdx.x & 31;
   double *E = ecache + (size_t)(threadIdx.x >> 5) * cache;
   const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t u = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; u < units;
-       u += warps) {
+  // a warp looks at up to 32 units at once for marked ones, so few that it
+  // still gets several such chunks
+  const int chunk = (int)min(max(units / (4 * warps), (uint64_t)1), (uint64_t)32);
+  uint64_t at = ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5) * chunk, first = 0;
+  unsigned marked = 0;
+  while (marked || at < units) {
     int n;
     uint8_t fallback;
+    if (!marked) {
+      bool mark = false;
+      if (lane < chunk && at + lane < units) {
+        const uint8_t *s = unit_of(codes, offsets, lengths, at + lane, mode, &n, &fallback);
+        mark = n >= kSegWindow && n <= kSegMaxLength && (s[0] & 128);
+      }
+      marked = __ballot_sync(0xffffffffu, mark);
+      first = at;
+      at += warps * chunk;
+      if (!marked) continue;
+    }
+    const uint64_t u = first + __ffs(marked) - 1;
+    marked &= marked - 1;
     uint8_t *s = unit_of(codes, offsets, lengths, u, mode, &n, &fallback);
-    if (n < kSegWindow || n > kSegMaxLength) continue;
-    if (!(s[0] & 128)) continue;
     __syncwarp();
     if (lane == 0) s[0] &= 127;
     __syncwarp();
@@ -515,20 +648,17 @@ __global__ void __launch_bounds__(kSegBlock)
     if (cached) {
       const int per = (m + 31) / 32, p0 = lane * per, p1 = min(p0 + per, m);
       if (p0 < p1) {
-        int comp[20], state[21];
-        seg_state(s + p0, kSegWindow, comp, state);
+        SegWindowCounts counts;
+        for (int i = p0; i < p0 + kSegWindow; ++i) {
+          const int k = seg_class(s[i]);
+          if (k >= 0) counts.add(k);
+        }
         for (int p = p0;; ++p) {
-          E[p] = seg_entropy(a, state);
+          E[p] = counts.entropy(tables, a.ln2);
           if (p + 1 >= p1) break;
           const int out = seg_class(s[p]), in = seg_class(s[p + kSegWindow]);
-          if (out >= 0) {
-            state_shrink(state, comp[out]);
-            --comp[out];
-          }
-          if (in >= 0) {
-            state_grow(state, comp[in]);
-            ++comp[in];
-          }
+          if (out >= 0) counts.remove(out);
+          if (in >= 0) counts.add(in);
         }
       }
       __syncwarp();
