@@ -773,41 +773,6 @@ __device__ __forceinline__ void emit_hit(const SeedArgs &a, uint32_t qid, uint32
 constexpr int kSeedBlock = 256;
 constexpr int kUnitsPerWarp = 256;
 
-// Items waiting in shared memory until 32 of them are there, one stack per
-// warp: a warp finds seeds, member work and hits with whatever lanes have
-// one, and walks or writes them 32 at a time.
-template <typename T>
-struct WarpStack {
-  static constexpr uint32_t kCapacity = 64;  // 31 waiting and 32 more
-  T *item;
-  uint32_t n = 0;  // the same on every lane
-  // the lanes with `have` add theirs (all lanes call it)
-  __device__ __forceinline__ void push(bool have, T v) {
-    const unsigned m = __ballot_sync(0xffffffffu, have);
-    if (have) item[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = v;
-    n += __popc(m);
-    __syncwarp();
-  }
-  // the newest 32 (fewer: all), one per lane; false on lanes without one
-  __device__ __forceinline__ bool pop(T *v) {
-    const uint32_t take = n < 32 ? n : 32, lane = threadIdx.x & 31;
-    n -= take;
-    if (lane < take) *v = item[n + lane];
-    __syncwarp();
-    return lane < take;
-  }
-  // pops into a global list: one atomic for the warp
-  __device__ __forceinline__ void flush(T *list, unsigned long long *count,
-                                        unsigned long long cap) {
-    const uint32_t take = n < 32 ? n : 32, lane = threadIdx.x & 31;
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(count, (unsigned long long)take);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    T v;
-    if (pop(&v) && base + lane < cap) list[base + lane] = v;
-  }
-};
-
 // Shared memory of a seed-search block: the window and walk tables and the
 // warps' stacks.
 struct SeedShared {

@@ -137,11 +137,12 @@ __device__ __forceinline__ bool ungapped_hit(const uint8_t *q, const uint8_t *d,
 constexpr int kWalkTableBytes = 64 * 32 * 4;
 constexpr int kWalkDelim = -32768;
 
-__device__ __forceinline__ void load_walk_table(int32_t *tbl, const int32_t *m32, int delim) {
+__device__ __forceinline__ void load_walk_table(int32_t *tbl, const int32_t *m, int delim,
+                                                int stride = 32) {
   for (int i = threadIdx.x; i < kWalkTableBytes / 4; i += blockDim.x) {
     const int a = i >> 6, x = i & 63, b = x ^ a;
     int v = 0;
-    if (x < 32) v = (a == delim || b == delim) ? kWalkDelim : m32[b * 32 + a];
+    if (x < 32) v = (a == delim || b == delim) ? kWalkDelim : m[b * stride + a];
     tbl[i] = v;
   }
 }

@@ -38,7 +38,8 @@ constexpr int kWindow = 32;           // residue pairs either side
 constexpr int kWalkMaxEntry = 127;
 constexpr int kWalkMaxCutoff = 127;
 constexpr int kWalkStop = -513;       // a delimiter's (doubled) entry
-constexpr int kWalkBias = 0x5000;     // keeps a half from borrowing
+constexpr uint32_t kWalkBias = 0x5000;       // keeps a half from borrowing
+constexpr uint32_t kWalkBiasExact = 0x6200;  // (over 31 steps of 256 more)
 constexpr int kWalkFlag = 0x400;      // set in a drop of at least cutoff
 
 // Score table: the doubled score of (query code a, database code b) at byte
@@ -51,11 +52,12 @@ __host__ __device__ __forceinline__ int window_entry(int a, int b, int score, in
 }
 
 // Fills the table; returns (on every thread) whether the matrix is admitted.
-__device__ __forceinline__ bool load_window_table(uint32_t tbl, const int32_t *m32, int delim) {
+__device__ __forceinline__ bool load_window_table(uint32_t tbl, const int32_t *m, int delim,
+                                                  int stride = 32) {
   bool fits = true;
   for (int i = threadIdx.x; i < 32 * 32; i += blockDim.x) {
     const int a = i >> 5, x = i & 31, b = a ^ x;
-    const int score = m32[b * 32 + a];
+    const int score = m[b * stride + a];
     fits = fits && score >= -kWalkMaxEntry && score <= kWalkMaxEntry;
     const int v = window_entry(a, b, score, delim);
     row_store(tbl + 256 * a + 4 * x, (uint32_t)v);
@@ -124,13 +126,22 @@ __host__ __device__ __forceinline__ uint32_t window_addmax(uint32_t a, uint32_t 
 #endif
 }
 
-// Whether the seed is settled as no hit; *steps then holds the residue pairs
-// its two walks examine.
-__host__ __device__ __forceinline__ bool walk_window(uint32_t tbl, const uint32_t q[16],
-                                                     const uint32_t d[16], int cutoff,
-                                                     int trigger, int *steps) {
+// Both walks over the window.  bests: the sum of the two sides' largest
+// (doubled) scores, from after a walk's end too unless kExact, where a score
+// falls by 256 a step from there on and so stays below its best.  steps and
+// delimiters (per half): the steps from the end on, and of those the ones
+// where a delimiter had been met.
+struct WindowWalk {
+  int bests;
+  int steps[2], delimiters[2];
+};
+
+template <bool kExact>
+__host__ __device__ __forceinline__ WindowWalk walk_both(uint32_t tbl, const uint32_t q[16],
+                                                         const uint32_t d[16], int cutoff) {
+  constexpr uint32_t bias = kExact ? kWalkBiasExact : kWalkBias;
   const uint32_t add = 0x10001u * (uint32_t)(kWalkFlag - 2 * cutoff);
-  uint32_t score = 0x10001u * kWalkBias;
+  uint32_t score = 0x10001u * bias;
   uint32_t best = score + add;  // best + add
   uint32_t flags = 0, sum = 0;
 #define GZB_WINDOW_PAIR(J)                                                       \
@@ -138,6 +149,7 @@ __host__ __device__ __forceinline__ bool walk_window(uint32_t tbl, const uint32_
     const uint32_t r = row_load_const(tbl + window_offset<3 - (J)>(xr, q[7 - k])); \
     const uint32_t f = row_load_const(tbl + window_offset<(J)>(xf, q[8 + k]) + 128); \
     score = score + r + f;                                                       \
+    if (kExact) score -= (flags >> 2) & (0x10001u * (kWalkFlag >> 2));           \
     best = window_addmax(score, add, best);                                      \
     flags = (flags | (best - score)) & (0x10001u * (kWalkFlag | 1));             \
     sum += flags;                                                                \
@@ -151,14 +163,70 @@ __host__ __device__ __forceinline__ bool walk_window(uint32_t tbl, const uint32_
     GZB_WINDOW_PAIR(3)
   }
 #undef GZB_WINDOW_PAIR
-  // steps from the end on (0: the walk goes on), and of those that a
-  // delimiter had been met
-  const int nr = (int)(sum & 0xffffu) / kWalkFlag, nf = (int)(sum >> 16) / kWalkFlag;
-  const int zr = (int)(sum & (kWalkFlag - 1)), zf = (int)((sum >> 16) & (kWalkFlag - 1));
-  const int bests = (int)(best & 0xffffu) + (int)(best >> 16) -
-                    2 * (int)((add & 0xffffu) + kWalkBias);
-  *steps = 2 * (kWindow + 1) - nr - nf - (zr == nr ? 1 : 0) - (zf == nf ? 1 : 0);
-  return nr > 0 && nf > 0 && bests <= 2 * trigger;
+  WindowWalk w;
+  w.steps[0] = (int)(sum & 0xffffu) / kWalkFlag;
+  w.steps[1] = (int)(sum >> 16) / kWalkFlag;
+  w.delimiters[0] = (int)(sum & (kWalkFlag - 1));
+  w.delimiters[1] = (int)((sum >> 16) & (kWalkFlag - 1));
+  w.bests = (int)(best & 0xffffu) + (int)(best >> 16) - 2 * (int)((add & 0xffffu) + bias);
+  return w;
 }
+
+// Whether the seed is settled as no hit; *steps then holds the residue pairs
+// its two walks examine.
+__host__ __device__ __forceinline__ bool walk_window(uint32_t tbl, const uint32_t q[16],
+                                                     const uint32_t d[16], int cutoff,
+                                                     int trigger, int *steps) {
+  const WindowWalk w = walk_both<false>(tbl, q, d, cutoff);
+  *steps = 2 * (kWindow + 1);
+  for (int i = 0; i < 2; ++i) *steps -= w.steps[i] + (w.delimiters[i] == w.steps[i] ? 1 : 0);
+  return w.steps[0] > 0 && w.steps[1] > 0 && w.bests <= 2 * trigger;
+}
+
+// 1: a hit (scores the walks reach sum to more than the trigger), 0: none
+// (both walks end), -1: open.
+__host__ __device__ __forceinline__ int walk_window_hit(uint32_t tbl, const uint32_t q[16],
+                                                        const uint32_t d[16], int cutoff,
+                                                        int trigger) {
+  const WindowWalk w = walk_both<true>(tbl, q, d, cutoff);
+  return w.bests > 2 * trigger ? 1 : w.steps[0] > 0 && w.steps[1] > 0 ? 0 : -1;
+}
+
+// Items waiting in shared memory until 32 of them are there, one stack per
+// warp: a warp finds seeds, member work and hits with whatever lanes have
+// one, and walks or writes them 32 at a time.
+#ifdef __CUDACC__
+template <typename T>
+struct WarpStack {
+  static constexpr uint32_t kCapacity = 64;  // 31 waiting and 32 more
+  T *item;
+  uint32_t n = 0;  // the same on every lane
+  // the lanes with `have` add theirs (all lanes call it)
+  __device__ __forceinline__ void push(bool have, T v) {
+    const unsigned m = __ballot_sync(0xffffffffu, have);
+    if (have) item[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = v;
+    n += __popc(m);
+    __syncwarp();
+  }
+  // the newest 32 (fewer: all), one per lane; false on lanes without one
+  __device__ __forceinline__ bool pop(T *v) {
+    const uint32_t take = n < 32 ? n : 32, lane = threadIdx.x & 31;
+    n -= take;
+    if (lane < take) *v = item[n + lane];
+    __syncwarp();
+    return lane < take;
+  }
+  // pops into a global list: one atomic for the warp
+  __device__ __forceinline__ void flush(T *list, unsigned long long *count,
+                                        unsigned long long cap) {
+    const uint32_t take = n < 32 ? n : 32, lane = threadIdx.x & 31;
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(count, (unsigned long long)take);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    T v;
+    if (pop(&v) && base + lane < cap) list[base + lane] = v;
+  }
+};
+#endif
 
 }  // namespace gzb

@@ -1,7 +1,8 @@
 """The seed search's window evaluation (csrc/gzb_walk.cuh) on the CPU: the
 same source compiled for the host, against the pair by pair walk.  Every seed
 it settles is no hit, with the walk's own number of residue pairs; a seed that
-could be a hit, or whose walk leaves the window, is never settled."""
+could be a hit, or whose walk leaves the window, is never settled.  Its exact
+form decides hits, too, and leaves open only walks that leave the window."""
 import ctypes as C
 import os
 import shutil
@@ -68,9 +69,10 @@ def test_settled_seeds(windows, cutoff, top, worst):
     trigger = 3 * cutoff
     settled = np.zeros(3000, np.int32)
     steps = np.zeros(3000, np.int32)
+    hits = np.zeros(3000, np.int32)
     p = lambda a: C.c_void_p(a.ctypes.data)  # noqa: E731
     windows.walk_windows(p(q), p(d), C.c_uint64(3000), p(qpos), p(dpos), p(m), delim, cutoff,
-                         trigger, p(settled), p(steps))
+                         trigger, p(settled), p(steps), p(hits))
     for i in range(3000):
         a, b = int(qpos[i]), int(dpos[i])
         rb, rn = _side(q, d, a - 1, b - 1, -1, m, delim, cutoff)
@@ -78,6 +80,9 @@ def test_settled_seeds(windows, cutoff, top, worst):
         if settled[i]:
             assert rb + fb <= trigger, i
             assert steps[i] == rn + fn, i
+            assert hits[i] == 0, i
+        # open only where a walk leaves the window
+        assert hits[i] == (rb + fb > trigger) or (hits[i] < 0 and max(rn, fn) >= 32), i
     assert settled.sum() > 0 or cutoff == 127  # (no walk of the wide X-drop ends in a window)
 
 
@@ -96,5 +101,5 @@ def test_blosum_seeds_are_settled(windows):
     steps = np.zeros(5000, np.int32)
     p = lambda a: C.c_void_p(a.ctypes.data)  # noqa: E731
     windows.walk_windows(p(q), p(d), C.c_uint64(5000), p(qpos), p(dpos), p(m), 25, 15, 41,
-                         p(settled), p(steps))
+                         p(settled), p(steps), None)
     assert settled.mean() > 0.9

@@ -5,10 +5,10 @@
 
 using namespace gzb;
 
-// settled[i], steps[i] of seeds (qpos[i], dpos[i])
+// settled[i], steps[i] and (unless null) hits[i] of seeds (qpos[i], dpos[i])
 extern "C" void walk_windows(const uint8_t *q, const uint8_t *d, uint64_t n, const uint32_t *qpos,
                              const uint32_t *dpos, const int32_t *m32, int delim, int cutoff,
-                             int trigger, int32_t *settled, int32_t *steps) {
+                             int trigger, int32_t *settled, int32_t *steps, int32_t *hits) {
   std::vector<uint32_t> memory(kWindowTableBytes / 4);
   row_host_memory = reinterpret_cast<char *>(memory.data());
   for (int a = 0; a < 32; ++a)
@@ -25,5 +25,6 @@ extern "C" void walk_windows(const uint8_t *q, const uint8_t *d, uint64_t n, con
     fetch_window(d + dpos[i], w);
     align_window(d + dpos[i], w, da);
     settled[i] = walk_window(0, qa, da, cutoff, trigger, &steps[i]) ? 1 : 0;
+    if (hits) hits[i] = walk_window_hit(0, qa, da, cutoff, trigger);
   }
 }
