@@ -1782,7 +1782,7 @@ struct gzb_engine {
   // build results step
   DBuf tb_redo;
   DBuf tb_cols, tb_band_off, tb_band, tb_ops_bytes, tb_ops_off, tb_rows, tb_rows_off, tb_ops,
-      tb_row_meta, tb_score, tb_p0, tb_p1, tb_out, tb_stats, tb_scratch;
+      tb_row_meta, tb_score, tb_p0, tb_p1, tb_out, tb_stats, tb_scratch, tb_order, tb_counters;
   uint64_t pred_n = 0;       // extensions with a prediction in epred (last run)
   DBuf enb;                  // per surviving hit: chained neighbours (cost feature)
   int tile[3][kTileParameters] = {
@@ -2036,7 +2036,7 @@ extern "C" int gzb_engine_destroy(gzb_engine *e) {
                  &e->tb_redo,
                  &e->tb_band, &e->tb_ops_bytes, &e->tb_ops_off, &e->tb_rows, &e->tb_rows_off,
                  &e->tb_ops, &e->tb_row_meta, &e->tb_score, &e->tb_p0, &e->tb_p1, &e->tb_out, &e->tb_stats,
-                 &e->tb_scratch};
+                 &e->tb_scratch, &e->tb_order, &e->tb_counters};
   for (DBuf *b : all) b->release();
   for (auto &g : e->graphs) cudaGraphExecDestroy(g.exec);
   e->graphs.clear();
@@ -3784,11 +3784,47 @@ extern "C" int gzb_engine_build_alignments(gzb_engine *e, uint32_t *counts,
   const uint64_t blocks = std::max<uint64_t>(
       1, std::min<uint64_t>(want, (uint64_t)sms * std::max(per_sm, 1)));
   GZB_TRY(e->tb_scratch.ensure(blocks * (kTbWarpBlock / 32) * kTbScratchBytes));
+  GZB_TRY(e->tb_counters.ensure(sizeof(TbCounters)));
+  TbCounters *ctr = e->tb_counters.as<TbCounters>();
+  GZB_CUDA(cudaMemsetAsync(ctr, 0, sizeof(TbCounters), s));
+  // more sides than warps: the longest first (their buckets and ranks in
+  // arrays that the warps fill later)
+  uint32_t *order = nullptr;
+  if (want > blocks && n_sides <= 0xffffffffull) {
+    GZB_TRY(e->tb_order.ensure(4 * n_sides));
+    order = e->tb_order.as<uint32_t>();
+    const unsigned grid = (unsigned)((n_sides + 255) / 256);
+    tb_rank_kernel<<<grid, 256, 0, s>>>(
+        a, n_sides, ctr->bucket_sides, e->tb_score.as<uint8_t>(), e->tb_p0.as<uint32_t>(),
+        e->tb_redo.as<uint8_t>(), e->tb_ops_bytes.as<uint64_t>(), e->tb_rows.as<uint64_t>());
+    GZB_CUDA(cudaGetLastError());
+    tb_order_kernel<<<grid, 256, 0, s>>>(n_sides, ctr->bucket_sides, e->tb_score.as<uint8_t>(),
+                                         e->tb_p0.as<uint32_t>(), order);
+    GZB_CUDA(cudaGetLastError());
+  }
   tb_side_warp_kernel<<<(unsigned)blocks, kTbWarpBlock, 0, s>>>(
       a, n_sides, e->tb_scratch.as<uint8_t>(), e->tb_score.as<int32_t>(),
       e->tb_p0.as<int32_t>(), e->tb_p1.as<int32_t>(), e->tb_stats.as<TbStats>(),
-      e->tb_ops_bytes.as<uint64_t>(), e->tb_rows.as<uint64_t>(), e->tb_redo.as<uint8_t>());
+      e->tb_ops_bytes.as<uint64_t>(), e->tb_rows.as<uint64_t>(), e->tb_redo.as<uint8_t>(), order,
+      ctr);
   GZB_CUDA(cudaGetLastError());
+  // nearly always no side is flagged: the results are joined and copied
+  // before the host knows, and again where one was
+  auto join = [&]() -> int {
+    tb_combine_kernel<<<grid1(n_slots, 128), 128, 0, s>>>(
+        a, n_slots, e->tb_score.as<int32_t>(), e->tb_p0.as<int32_t>(), e->tb_p1.as<int32_t>(),
+        e->tb_stats.as<TbStats>(), e->tb_out.as<gzb_alignment>());
+    GZB_CUDA(cudaGetLastError());
+    GZB_CUDA(cudaMemcpyAsync(counts, e->counts.p, 4 * (uint64_t)e->nq, cudaMemcpyDeviceToHost, s));
+    GZB_CUDA(cudaMemcpyAsync(alignments, e->tb_out.p, sizeof(gzb_alignment) * n_slots,
+                             cudaMemcpyDeviceToHost, s));
+    return GZB_OK;
+  };
+  uint32_t redo = 0;
+  GZB_TRY(join());
+  GZB_CUDA(cudaMemcpyAsync(&redo, &ctr->redo, 4, cudaMemcpyDeviceToHost, s));
+  GZB_CUDA(cudaStreamSynchronize(s));
+  if (redo == 0) return GZB_OK;
   // the flagged sides' bands (global memory) and storage sizes
   GZB_TRY(e->tb_cols.ensure(8 * (n_sides + 1)));
   tb_band_kernel<<<grid1(n_sides, 256), 256, 0, s>>>(a, n_sides, e->tb_redo.as<uint8_t>(),
@@ -3813,13 +3849,7 @@ extern "C" int gzb_engine_build_alignments(gzb_engine *e, uint32_t *counts,
       e->tb_row_meta.as<uint32_t>(), e->tb_score.as<int32_t>(), e->tb_p0.as<int32_t>(),
       e->tb_p1.as<int32_t>(), e->tb_stats.as<TbStats>(), e->tb_redo.as<uint8_t>());
   GZB_CUDA(cudaGetLastError());
-  tb_combine_kernel<<<grid1(n_slots, 128), 128, 0, s>>>(
-      a, n_slots, e->tb_score.as<int32_t>(), e->tb_p0.as<int32_t>(), e->tb_p1.as<int32_t>(),
-      e->tb_stats.as<TbStats>(), e->tb_out.as<gzb_alignment>());
-  GZB_CUDA(cudaGetLastError());
-  GZB_CUDA(cudaMemcpyAsync(counts, e->counts.p, 4 * (uint64_t)e->nq, cudaMemcpyDeviceToHost, s));
-  GZB_CUDA(cudaMemcpyAsync(alignments, e->tb_out.p, sizeof(gzb_alignment) * n_slots,
-                           cudaMemcpyDeviceToHost, s));
+  GZB_TRY(join());
   GZB_CUDA(cudaStreamSynchronize(s));
   return GZB_OK;
 }

@@ -527,6 +527,61 @@ __device__ TbStats tb_walk_stats(const uint8_t *ops, const uint32_t *meta, int i
   return st;
 }
 
+// The sides in order of the presearch's rows, the longest first, in buckets
+// of a quarter octave: with more sides than warps one that starts last and
+// runs long leaves the rest of the device idle.  Static strides over the
+// sides of 1,000 queries x 20,000 proteins: 3.1 ms, the busiest SM twice the
+// average; in this order 2.5.  A side's bucket and rank within it; sides
+// without a result are finished here.
+__global__ void tb_rank_kernel(TbArgs a, uint64_t n_sides, uint32_t *bucket_sides,
+                               uint8_t *bucket, uint32_t *rank, uint8_t *redo,
+                               uint64_t *ops_bytes, uint64_t *rows) {
+  __shared__ uint32_t count[kTbBuckets], base[kTbBuckets];
+  if (threadIdx.x < kTbBuckets) count[threadIdx.x] = 0;
+  __syncthreads();
+  const uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  int k = -1;
+  uint32_t at = 0;
+  if (s < n_sides) {
+    if (side_of(a, s).active) {
+      const gzb_result r = a.results[s >> 1];
+      const uint32_t reach = (s & 1) ? r.end_d - r.hit_d : r.hit_d - r.start_d;
+      // (a side's X-drop goes on past the presearch's)
+      const uint32_t e = 64 + (reach > (1u << 21) - 65 ? (1u << 21) - 65 : reach);
+      const int octave = 31 - __clz((int)e);
+      k = kTbBuckets - 1 - ((octave - 6) * 4 + (int)((e >> (octave - 2)) & 3));
+      at = atomicAdd(&count[k], 1u);
+    } else {
+      redo[s] = 0;
+      ops_bytes[s] = 0;
+      rows[s] = 0;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < kTbBuckets && count[threadIdx.x])
+    base[threadIdx.x] = atomicAdd(&bucket_sides[threadIdx.x], count[threadIdx.x]);
+  __syncthreads();
+  if (s < n_sides) {
+    bucket[s] = (uint8_t)(k < 0 ? kTbBuckets : k);
+    if (k >= 0) rank[s] = base[k] + at;
+  }
+}
+
+__global__ void tb_order_kernel(uint64_t n_sides, const uint32_t *bucket_sides,
+                                const uint8_t *bucket, const uint32_t *rank, uint32_t *order) {
+  __shared__ uint32_t first[kTbBuckets];
+  if (threadIdx.x == 0) {
+    uint32_t n = 0;
+    for (int k = 0; k < kTbBuckets; ++k) {
+      first[k] = n;
+      n += bucket_sides[k];
+    }
+  }
+  __syncthreads();
+  const uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (s < n_sides && bucket[s] < kTbBuckets) order[first[bucket[s]] + rank[s]] = (uint32_t)s;
+}
+
 // One warp per side runs the DP with its ops and row table into the warp's
 // own scratch (kTbScratchOps bytes, kTbScratchRows rows), where up to 32
 // sides gather; then each lane walks one of them (PickOptimalPath and
@@ -534,11 +589,13 @@ __device__ TbStats tb_walk_stats(const uint8_t *ops, const uint32_t *meta, int i
 // reused.  A side the warp cannot run exactly (X-drop >= 1024, a band wider
 // than kTbMaxBand) or whose storage outgrows an empty scratch is
 // flagged in `redo` with its sizes left to the thread kernels; the others
-// get zero sizes.
+// get zero sizes.  `order` (or null: side after side): the sides to run, the
+// next of them to whichever warp is free.
 __global__ void __launch_bounds__(kTbWarpsPerBlock * 32, 4)
     tb_side_warp_kernel(TbArgs a, uint64_t n_sides, uint8_t *scratch, int32_t *side_score,
                         int32_t *side_p0, int32_t *side_p1, TbStats *stats, uint64_t *ops_bytes,
-                        uint64_t *rows, uint8_t *redo) {
+                        uint64_t *rows, uint8_t *redo, const uint32_t *order,
+                        TbCounters *counters) {
   __shared__ int sm[kMatrixStride * kMatrixStride];
   __shared__ TbBand bands[kTbWarpsPerBlock];
   load_matrix(sm, a.matrix32, 32, 32);  // the 32 x 32 device matrix
@@ -566,8 +623,21 @@ __global__ void __launch_bounds__(kTbWarpsPerBlock * 32, 4)
     meta_pos = 0;
     nacc = 0;
   };
-  for (uint64_t s = blockIdx.x * (uint64_t)kTbWarpsPerBlock + warp; s < n_sides;
-       s += (uint64_t)gridDim.x * kTbWarpsPerBlock) {
+  uint64_t todo = n_sides;
+  if (order) {
+    static_assert(kTbBuckets == 64, "two buckets a lane");
+    todo = __reduce_add_sync(0xffffffffu,
+                             counters->bucket_sides[lane] + counters->bucket_sides[lane + 32]);
+  }
+  uint64_t at = blockIdx.x * (uint64_t)kTbWarpsPerBlock + warp;
+  for (;; at += (uint64_t)gridDim.x * kTbWarpsPerBlock) {
+    if (order) {
+      uint32_t next = 0;
+      if (lane == 0) next = atomicAdd(&counters->next, 1u);
+      at = __shfl_sync(0xffffffffu, next, 0);
+    }
+    if (at >= todo) break;
+    const uint64_t s = order ? order[at] : at;
     const TbSide t = side_of(a, s);
     bool ok = !t.active;
     if (t.active && a.cutoff < 1024) {
@@ -602,6 +672,7 @@ __global__ void __launch_bounds__(kTbWarpsPerBlock * 32, 4)
     }
     if (lane == 0) {
       redo[s] = ok ? 0 : 1;
+      if (!ok) atomicAdd(&counters->redo, 1u);
       ops_bytes[s] = 0;
       rows[s] = 0;
     }

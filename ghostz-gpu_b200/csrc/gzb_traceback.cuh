@@ -38,6 +38,19 @@ constexpr uint64_t kTbScratchOps = 256 * 1024;
 constexpr uint32_t kTbScratchRows = 8192;
 constexpr uint64_t kTbScratchBytes = kTbScratchOps + 8ull * kTbScratchRows;
 
+// zeroed before the kernels that order and run the sides
+constexpr int kTbBuckets = 64;
+struct TbCounters {
+  uint32_t bucket_sides[kTbBuckets];  // sides in a bucket of the order
+  uint32_t next;                      // sides handed out
+  uint32_t redo;                      // sides left to the thread kernels
+};
+
+__global__ void tb_rank_kernel(TbArgs a, uint64_t n_sides, uint32_t *bucket_sides,
+                               uint8_t *bucket, uint32_t *rank, uint8_t *redo,
+                               uint64_t *ops_bytes, uint64_t *rows);
+__global__ void tb_order_kernel(uint64_t n_sides, const uint32_t *bucket_sides,
+                                const uint8_t *bucket, const uint32_t *rank, uint32_t *order);
 __global__ void tb_band_kernel(TbArgs a, uint64_t n_sides, const uint8_t *redo,
                                uint64_t *band_cols);
 // warps per block of the one-warp-per-side kernel
@@ -45,7 +58,8 @@ constexpr int kTbWarpBlock = 8 * 32;
 __global__ void tb_side_warp_kernel(TbArgs a, uint64_t n_sides, uint8_t *scratch,
                                     int32_t *side_score, int32_t *side_p0, int32_t *side_p1,
                                     TbStats *stats, uint64_t *ops_bytes, uint64_t *rows,
-                                    uint8_t *redo);
+                                    uint8_t *redo, const uint32_t *order,
+                                    TbCounters *counters);
 __global__ void tb_count_kernel(TbArgs a, uint64_t n_sides, const uint64_t *band_off,
                                 int2 *band, uint64_t *ops_bytes, uint64_t *rows,
                                 const uint8_t *redo);
