@@ -221,7 +221,8 @@ struct TbBand {
 //    in at or above the threshold t = max - X-drop, or some cell could open
 //    one (score - gap >= t).  Gaps below t keep no cell, start no path
 //    operation and grow no band.
-//  * the running maximum's scan where a cell exceeds it.
+//  * the running maximum's scan where cells raise it more than once: with
+//    one that raises it, it is the old one before and the new one from there.
 // The gap is not reset behind a pruned cell, for the ops as for the
 // decisions: where that differs from the reference's, the gap is below t.  A
 // kept cell's score is not, so its op is the same; an extension flag is read
@@ -353,18 +354,24 @@ __device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, 
       }
       const int raw = imax(G, Fl);
       int Mrow = maxs;
-      if (__any_sync(full, active && raw > maxs)) {
-        int R = active ? raw : kNegBig;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int tv = __shfl_up_sync(full, R, o);
-          if (lane >= o) R = imax(R, tv);
-        }
-        Mrow = imax(maxs, R);
+      const unsigned up = __ballot_sync(full, active && raw > maxs);
+      if (up) {
+        const int now = __reduce_max_sync(full, active ? raw : kNegBig);
         // the new maximum: first column reaching it
-        maxs = __shfl_sync(full, R, 31);
-        const unsigned hitm = __ballot_sync(full, active && raw == maxs);
-        mp0 = (cs + __ffs(hitm) - 2) * inc;
+        const int at = __ffs(__ballot_sync(full, active && raw == now)) - 1;
+        if (at == __ffs(up) - 1) {
+          if (lane >= at) Mrow = now;
+        } else {
+          int R = active ? raw : kNegBig;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int tv = __shfl_up_sync(full, R, o);
+            if (lane >= o) R = imax(R, tv);
+          }
+          Mrow = imax(maxs, R);
+        }
+        maxs = now;
+        mp0 = (cs + at - 1) * inc;
         mp1 = (int)r * inc;
       }
       const bool keep = active && Mrow - raw <= cutoff;
@@ -400,10 +407,12 @@ __device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, 
       be = last_kept + 1;
     } else {
       // grow along the horizontal gap while F >= max - cutoff
-      const long long room = (long long)F - ((long long)maxs - cutoff);
+      const int room = F - (maxs - cutoff);
       if (room >= 0) {
-        const long long kk = ge == 0 ? kFar : room / ge + 1;
-        const int k1 = (int)(kk > kFar ? kFar : kk);
+        // floor(room / ge) + 1 columns
+        const unsigned grown = __ballot_sync(full, lane * ge <= room);
+        int k1 = __popc(grown);
+        if (grown == full) k1 = ge == 0 ? kFar : (int)((unsigned)room / (unsigned)ge) + 1;
         see(be + imin(k1, W));
         const int k = imin(k1, delim_at - be);
         if (be + k - bs > W) return false;
