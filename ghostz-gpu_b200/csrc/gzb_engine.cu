@@ -779,32 +779,37 @@ struct SeedShared {
   uint32_t window[kWindowTableBytes / 4];
   int32_t walk[kWalkTableBytes / 4];
   uint4 found[kSeedBlock / 32][WarpStack<uint4>::kCapacity];
-  uint2 open[kSeedBlock / 32][WarpStack<uint2>::kCapacity];
+  uint4 open[kSeedBlock / 32][WarpStack<uint4>::kCapacity];
+  uint2 whole[kSeedBlock / 32][WarpStack<uint2>::kCapacity];
   uint2 member[kSeedBlock / 32][WarpStack<uint2>::kCapacity];
   uint64_t hit[kSeedBlock / 32][WarpStack<uint64_t>::kCapacity];
 };
 
 // The walks of the seeds a warp finds.  Each seed's window is evaluated
-// first (gzb_walk.cuh: no branches, every lane the same length); the one in
-// ten that this leaves open is walked pair by pair, again 32 together.
+// first (gzb_walk.cuh: no branches, every lane the same length); the walks of
+// the one in ten that this leaves open go on from there, and the few that
+// come near the trigger are walked pair by pair from the seed, each kind 32
+// together.
 //
 // One walk after another per lane instead (each warp waiting for its longest
 // walk, lanes idle where the distance filter had refused) ran 14.6 of 32
 // lanes an instruction, this 27.  Seed and member kernels together, 1.04 G
-// seeds of 10,000 queries x 1,500,000 proteins: 58.2 -> 47.8 ms; 82 M seeds
-// of 2,000 x 400,000: 5.1 -> 4.3 ms.  What is left (2,000 x 400,000): ALU
-// pipe 63 %, L1 wavefronts 62 %, issue 57 %, 3.4 cycles an instruction
-// waiting for global loads; of the 47.8 ms the search for seeds takes 10,
-// the windows' loads 20, their evaluation 10, the open walks 9.  Three
-// blocks an SM: four (64 registers) 50.6 ms; the windows of the next seeds
-// fetched ahead into registers 55 ms (two blocks); prefetched into L2 54.6.
+// seeds of 10,000 queries x 1,500,000 proteins: 58.2 -> 45.5 ms (48.2 with
+// open walks done whole); 82 M seeds of 2,000 x 400,000: 5.1 -> 4.1 ms.  What
+// is left (2,000 x 400,000, open walks whole): ALU pipe 63 %, L1 wavefronts
+// 62 %, issue 57 %, 3.4 cycles an instruction waiting for global loads; of
+// the 48 ms the search for seeds took 10, the windows' loads 20, their
+// evaluation 10, the open walks 9.  Three blocks an SM: four (64 registers)
+// 50.6 ms; the windows of the next seeds fetched ahead into registers 55 ms
+// (two blocks); prefetched into L2 54.6.
 struct SeedWalker {
   const SeedArgs &a;
   uint32_t window;   // table addresses
   const char *walk;
   bool fits;         // the matrix (window tables hold entries up to 127)
   WarpStack<uint4> found;     // (database position, entry, its position, cutoff and trigger)
-  WarpStack<uint2> open;      // (database position, entry)
+  WarpStack<uint4> open;      // (database position, entry, the window's sides)
+  WarpStack<uint2> whole;     // (database position, entry) of whole walks
   WarpStack<uint64_t> hit;    // packed hit keys
   // a thread's counts stay far below 2^32 (that many walk steps would take
   // one thread seconds)
@@ -817,6 +822,7 @@ struct SeedWalker {
     fits = load_window_table(window, a.matrix32, a.p.delimiter);
     found.item = sh.found[threadIdx.x >> 5];
     open.item = sh.open[threadIdx.x >> 5];
+    whole.item = sh.whole[threadIdx.x >> 5];
     hit.item = sh.hit[threadIdx.x >> 5];
   }
 
@@ -830,6 +836,7 @@ struct SeedWalker {
   __device__ __forceinline__ void finish() {
     if (found.n) run_found();
     while (open.n) run_open();
+    while (whole.n) run_whole();
     while (hit.n) hit.flush(a.hits, a.hit_count, a.hit_cap);
   }
 
@@ -837,6 +844,7 @@ struct SeedWalker {
     uint4 v = make_uint4(0, 0, 0, 0);
     const bool have = found.pop(&v);
     bool settled = false;
+    uint32_t side[2] = {kSideUnknown, 0};
     if (have) {
       ++n_seed;
       const int cutoff = (int)(v.w >> 16), trigger = (int)(int16_t)(v.w & 0xffffu);
@@ -849,19 +857,35 @@ struct SeedWalker {
         align_window(qs, qw, q);
         align_window(ds, dw, d);
         int steps;
-        settled = walk_window(window, q, d, cutoff, trigger, &steps);
+        settled = walk_window(window, q, d, cutoff, trigger, &steps, side);
         if (settled) n_steps += (uint32_t)steps;
       }
     }
-    open.push(have && !settled, make_uint2(v.x, v.y));
+    open.push(have && !settled, make_uint4(v.x, v.y, side[0], side[1]));
     if (open.n >= 32) run_open();
   }
 
   __device__ __forceinline__ void run_open() {
+    uint4 v = make_uint4(0, 0, 0, 0);
+    const bool have = open.pop(&v);
+    bool settled = false;
+    if (have) {
+      const uint32_t ct = a.L.entry_ct[v.y], side[2] = {v.z, v.w};
+      int steps = 0;
+      settled = walk_on(a.q + a.L.entry_cpos[v.y], a.db + v.x, walk,
+                                       (int)(ct >> 16), (int)(int16_t)(ct & 0xffffu), side,
+                                       &steps);
+      if (settled) n_steps += (uint32_t)steps;
+    }
+    whole.push(have && !settled, make_uint2(v.x, v.y));
+    if (whole.n >= 32) run_whole();
+  }
+
+  __device__ __forceinline__ void run_whole() {
     uint2 v = make_uint2(0, 0);
     bool is_hit = false;
     uint64_t key = 0;
-    if (open.pop(&v)) {
+    if (whole.pop(&v)) {
       const uint32_t ct = a.L.entry_ct[v.y], cpos = a.L.entry_cpos[v.y];
       int steps = 0;
       is_hit = walk_hit(a.q + cpos, a.db + v.x, walk, (int)(ct >> 16),

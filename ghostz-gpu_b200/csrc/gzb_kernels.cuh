@@ -194,10 +194,10 @@ __device__ __forceinline__ void load_walk_words(WalkWords<INC> &ww, const uint8_
 template <int INC>
 __device__ __forceinline__ int walk_side_words(const WalkWords<INC> &A, const WalkWords<INC> &B,
                                                const char *tbl, int cutoff, int stop_above,
-                                               int *steps) {
+                                               int *steps, int score, int best) {
   constexpr int K = kWalkPrefetch;
   const uint32_t sha = A.sh, shb = B.sh;
-  int score = 0, best = 0, n = 0;
+  int n = 0;
   uint32_t rx4 = 0, rqa = 0;  // the chunk the walk ends in
 #define GZB_WALK_V(J, X4, QA) \
   (*(const int32_t *)(tbl + walk_offset<(INC > 0 ? (J) : 3 - (J))>(X4, QA)))
@@ -299,7 +299,7 @@ done:
 // from s0[0]/s1[0] (query/database) stepping by INC: returns the best prefix
 // score, stopping at the X-drop (best - score >= cutoff, cutoff >= 1), at a
 // delimiter, or once the best exceeds stop_above.  The reference's
-// (best, run) pair is (best, score - best) here.  Reads four residue pairs
+// (best, run) pair is (best, score - best) here; a walk may go on from one.  Reads four residue pairs
 // per pair of aligned 32-bit words.  The first kWalkPrefetch chunks' words
 // are loaded together up front (most walks end inside them, so a walk waits
 // for one round of loads instead of one per chunk); a longer walk goes on
@@ -308,11 +308,11 @@ done:
 template <int INC>
 __device__ __forceinline__ int walk_side(const uint8_t *s0, const uint8_t *s1,
                                          const char *tbl, int cutoff, int stop_above,
-                                         int *steps) {
+                                         int *steps, int score = 0, int best = 0) {
   WalkWords<INC> A, B;
   load_walk_words(A, s0);
   load_walk_words(B, s1);
-  return walk_side_words(A, B, tbl, cutoff, stop_above, steps);
+  return walk_side_words(A, B, tbl, cutoff, stop_above, steps, score, best);
 }
 
 // Whether the X-drop walk from s0[0]/s1[0] stepping by INC survives its

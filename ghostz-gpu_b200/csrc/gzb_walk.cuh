@@ -9,7 +9,8 @@
 // 32 pairs of both sides for every seed: where both walks end and even the
 // windows' largest scores (an upper bound of the bests) do not exceed the
 // trigger, the seed is settled, with the exact number of pairs the walks
-// examined; the other seeds are left to walk_hit, 32 of them together.
+// examined; the other seeds' walks go on from their windows' ends (walk_on),
+// 32 of them together, and those near the trigger are left to walk_hit.
 //
 // Both sides are computed in one word, reverse in the low half and forward in
 // the high half, scores doubled.  Per pair of pairs: two table words (the
@@ -133,7 +134,20 @@ __host__ __device__ __forceinline__ uint32_t window_addmax(uint32_t a, uint32_t 
 // where a delimiter had been met.
 struct WindowWalk {
   int bests;
+  int best[2], score[2];  // per side, doubled (score: at the window's end)
   int steps[2], delimiters[2];
+
+  // the residue pairs side i's walk examines, if it ends in the window
+  __host__ __device__ __forceinline__ int pairs(int i) const {
+    return kWindow + 1 - steps[i] - (delimiters[i] == steps[i] ? 1 : 0);
+  }
+  __host__ __device__ __forceinline__ bool ended(int i) const { return steps[i] > 0; }
+  // side i in a word: an ended walk's pairs and (an upper bound of) its
+  // best, an open one's best and its drop below it
+  __host__ __device__ __forceinline__ uint32_t side(int i) const {
+    return ended(i) ? 0x80000000u | (uint32_t)((best[i] + 1) >> 1) << 16 | (uint32_t)pairs(i)
+                    : (uint32_t)(best[i] >> 1) << 16 | (uint32_t)((best[i] - score[i]) >> 1);
+  }
 };
 
 template <bool kExact>
@@ -168,20 +182,54 @@ __host__ __device__ __forceinline__ WindowWalk walk_both(uint32_t tbl, const uin
   w.steps[1] = (int)(sum >> 16) / kWalkFlag;
   w.delimiters[0] = (int)(sum & (kWalkFlag - 1));
   w.delimiters[1] = (int)((sum >> 16) & (kWalkFlag - 1));
-  w.bests = (int)(best & 0xffffu) + (int)(best >> 16) - 2 * (int)((add & 0xffffu) + bias);
+  const int zero = (int)((add & 0xffffu) + bias);
+  w.best[0] = (int)(best & 0xffffu) - zero;
+  w.best[1] = (int)(best >> 16) - zero;
+  w.score[0] = (int)(score & 0xffffu) - (int)bias;
+  w.score[1] = (int)(score >> 16) - (int)bias;
+  w.bests = w.best[0] + w.best[1];
   return w;
 }
 
 // Whether the seed is settled as no hit; *steps then holds the residue pairs
-// its two walks examine.
+// its two walks examine.  If not, side[0] and side[1] (reverse and forward)
+// say where its walks are.
 __host__ __device__ __forceinline__ bool walk_window(uint32_t tbl, const uint32_t q[16],
                                                      const uint32_t d[16], int cutoff,
-                                                     int trigger, int *steps) {
+                                                     int trigger, int *steps, uint32_t side[2]) {
   const WindowWalk w = walk_both<false>(tbl, q, d, cutoff);
-  *steps = 2 * (kWindow + 1);
-  for (int i = 0; i < 2; ++i) *steps -= w.steps[i] + (w.delimiters[i] == w.steps[i] ? 1 : 0);
-  return w.steps[0] > 0 && w.steps[1] > 0 && w.bests <= 2 * trigger;
+  *steps = w.pairs(0) + w.pairs(1);
+  side[0] = w.side(0);
+  side[1] = w.side(1);
+  return w.ended(0) && w.ended(1) && w.bests <= 2 * trigger;
 }
+
+#ifdef __CUDACC__
+constexpr uint32_t kSideUnknown = 0xffffffffu;  // no window: the whole walk is to do
+
+// The walks of a seed that its window leaves open, from the window's ends:
+// true if it is no hit, with the pairs that both walks examine.  False where
+// a walk could have stopped at the trigger, which walk_hit settles.
+__device__ __forceinline__ bool walk_on(const uint8_t *q, const uint8_t *d, const char *tbl,
+                                        int cutoff, int trigger, const uint32_t side[2],
+                                        int *steps) {
+  int n = 0, best[2];
+  for (int i = 0; i < 2; ++i) {
+    best[i] = (int)((side[i] >> 16) & 0x7fffu);
+    n += side[i] >> 31 ? (int)(side[i] & 0xffffu) : kWindow;
+  }
+  if (side[0] == kSideUnknown || best[0] + best[1] > trigger) return false;
+  if (!(side[0] >> 31))
+    best[0] = walk_side<-1>(q - 1 - kWindow, d - 1 - kWindow, tbl, cutoff,
+                               trigger - best[1], &n, best[0] - (int)(side[0] & 0xffffu), best[0]);
+  if (best[0] + best[1] > trigger) return false;
+  if (!(side[1] >> 31))
+    best[1] = walk_side<1>(q + kWindow, d + kWindow, tbl, cutoff, trigger - best[0], &n,
+                              best[1] - (int)(side[1] & 0xffffu), best[1]);
+  *steps = n;
+  return best[0] + best[1] <= trigger;
+}
+#endif
 
 // 1: a hit (scores the walks reach sum to more than the trigger), 0: none
 // (both walks end), -1: open.

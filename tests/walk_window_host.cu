@@ -24,7 +24,8 @@ extern "C" void walk_windows(const uint8_t *q, const uint8_t *d, uint64_t n, con
     align_window(q + qpos[i], w, qa);
     fetch_window(d + dpos[i], w);
     align_window(d + dpos[i], w, da);
-    settled[i] = walk_window(0, qa, da, cutoff, trigger, &steps[i]) ? 1 : 0;
+    uint32_t side[2];
+    settled[i] = walk_window(0, qa, da, cutoff, trigger, &steps[i], side) ? 1 : 0;
     if (hits) hits[i] = walk_window_hit(0, qa, da, cutoff, trigger);
   }
 }
