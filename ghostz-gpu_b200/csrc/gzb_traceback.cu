@@ -234,7 +234,8 @@ struct TbBand {
 // All scans of every chunk, and the loads where their values were needed,
 // took (the whole kernel) 4.2 ms on the alignments of 1,000 queries x 20,000
 // proteins, which long homologs dominate, and 18.7 ms on those of 30,000
-// reads x 400,000; this takes 3.2 and 14.0 ms.
+// reads x 400,000; this took 3.2 and 14.0 ms, and 2.35 and 11.4 with the order
+// of tb_rank_kernel and the maximum's scan left out.
 __device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, TbBand &band,
                                uint8_t *ops, uint32_t *row_meta, uint64_t ops_cap,
                                uint32_t rows_cap, uint64_t *ops_bytes, uint32_t *rows,
