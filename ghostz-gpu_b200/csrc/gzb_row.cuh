@@ -321,6 +321,14 @@ __host__ __device__ __forceinline__ void row_new_group(const Band &band, RowExt 
   row_store4(band.group(g), RowGroup{{kEmptyCell, kEmptyCell, kEmptyCell, kEmptyCell}});
 }
 
+// The band ends at the query's end: its last column's best score is no
+// diagonal for the delimiter's column, which its group evaluates with it.
+template <class Band>
+__host__ __device__ __forceinline__ void row_end_diagonal(const Band &band, int last) {
+  const uint32_t a = band.column(last);
+  row_store(a, (row_load(a) & 0xffff0000u) | (kEmptyCell & 0xffffu));
+}
+
 // Row -1 (src/gapped_extender.cpp:345-364): the gap row along the query.
 template <int W, int STRIDE>
 __host__ __device__ __forceinline__ int row_init(const GappedJob &job,
@@ -370,6 +378,7 @@ __host__ __device__ __forceinline__ int row_init(const GappedJob &job,
     if (4 * x.groups > end) {
       x.bs = 0;
       x.be = end < x.delim_at ? end + 1 : end;  // the sentinel column
+      if (end >= x.delim_at) row_end_diagonal(band, end - 1);
       break;
     }
     if (x.groups == Band::kGroups) return kLaneOverflow;
@@ -521,10 +530,9 @@ __host__ __device__ __forceinline__ int row_step(const GappedJob &job, uint32_t 
     if ((edge >> 2) >= x.groups || ((x.be - 1) >> 2) - (x.bs >> 2) >= Band::kGroups) {
       st = kLaneOverflow;
     } else if (edge >= x.delim_at) {
-      // no sentinel: the next column has no diagonal
+      // no sentinel
       x.be = last + 1;
-      const uint32_t a = band.column(last);
-      row_store(a, (row_load(a) & 0xffff0000u) | (kEmptyCell & 0xffffu));
+      row_end_diagonal(band, last);
     }
   }
   row_meet();

@@ -131,3 +131,31 @@ def test_admitted_parameters(rows, go, ge, cutoff, admitted):
     st, _ = _run(rows, 64, q, q0, q, q0, 25, go, ge, cutoff, False, matrix)
     fits = -1 + ge < 1024 - cutoff
     assert (st != -1) == (admitted and fits)
+
+
+# The first row's columns reach the query's end where a gap is cheap: the
+# delimiter's column is no cell, whatever the score table holds for its byte
+# (codes from 32 on read a neighbouring row's entries, a delimiter below the
+# matrix's side its own).
+@pytest.mark.parametrize("delim", [19, 25, 31, 34, 50, 63, 64, 100, 200, 255])
+@pytest.mark.parametrize("go,ge,cutoff", [(0, 1, 30), (1, 1, 30), (2, 3, 60), (4, 0, 10)])
+def test_delimiter_column_is_no_cell(rows, oracle, delim, go, ge, cutoff):
+    rng = np.random.default_rng(delim * 100 + go + ge)
+    matrix = P.blosum62()[:20, :20]
+    matrix[:, 19] = matrix[19, :] = 9
+    done = 0
+    for n in list(range(1, 14)) * 12:
+        letters = 19
+        a, b = (rng.integers(0, letters, k).astype(np.uint8) for k in (n, int(rng.integers(1, 30))))
+        q, q0 = _buffer(rng, a, delim, letters)
+        d, d0 = _buffer(rng, b, delim, letters)
+        params = P.make_params(matrix=matrix, gap_open=go, gap_extension=ge)
+        params["delimiter"] = delim
+        for rev in (False, True):
+            i, j = (len(a) - 1, len(b) - 1) if rev else (0, 0)
+            st, got = _run(rows, 32, q, q0 + i, d, d0 + j, delim, go, ge, cutoff, rev, matrix)
+            if st == 1:
+                assert got == oracle.gapped_one_side(params, q, q0 + i, d, d0 + j, rev, cutoff), \
+                    (n, rev)
+                done += 1
+    assert done > 100
