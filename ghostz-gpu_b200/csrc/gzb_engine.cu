@@ -1773,6 +1773,9 @@ namespace {
 // copy pieces into it and queue their transfers.  The driver's own copy is one
 // thread's; 72 MB took 6.0 ms through it and take 2.4 this way.  One per
 // engine, made at its first large upload, given back with the engine.
+// The transfers run on a stream of the staging's own, which starts after the
+// work queued on the caller's and which that waits for: the caller's handle
+// can mean another stream in another thread (cudaStreamPerThread).
 class Staging {
  public:
   static constexpr uint64_t kPiece = 1 << 20;
@@ -1781,12 +1784,12 @@ class Staging {
 
   // queues the copy of n bytes on s; src may change once this returns
   cudaError_t copy(void *dst, const void *src, uint64_t n, int device, cudaStream_t s) {
-    cudaPointerAttributes attr;
-    if (n < kLeast || cudaPointerGetAttributes(&attr, src) != cudaSuccess ||
-        attr.type != cudaMemoryTypeUnregistered || !make()) {
+    if (n < kLeast || !pageable(src) || capturing(s) || !make()) {
       cudaGetLastError();
       return cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, s);
     }
+    cudaError_t r = follow(stream_, s);
+    if (r != cudaSuccess) return r;
     std::atomic<uint64_t> next{0};
     std::atomic<int> error{(int)cudaSuccess};
     auto work = [&](int t) {
@@ -1800,8 +1803,8 @@ class Staging {
         if ((r = cudaEventSynchronize(done_[b])) != cudaSuccess) break;
         std::memcpy(memory_ + b * kPiece, (const uint8_t *)src + at, m);
         r = cudaMemcpyAsync((uint8_t *)dst + at, memory_ + b * kPiece, m,
-                            cudaMemcpyHostToDevice, s);
-        if (r == cudaSuccess) r = cudaEventRecord(done_[b], s);
+                            cudaMemcpyHostToDevice, stream_);
+        if (r == cudaSuccess) r = cudaEventRecord(done_[b], stream_);
       }
       if (r != cudaSuccess) error = (int)r;
     };
@@ -1813,29 +1816,54 @@ class Staging {
     }
     work(0);
     for (std::thread &t : others) t.join();
-    return (cudaError_t)error.load();
+    r = follow(s, stream_);  // (after an error too: pieces may be under way)
+    return error.load() != (int)cudaSuccess ? (cudaError_t)error.load() : r;
   }
 
   void release() {
+    if (stream_) cudaStreamSynchronize(stream_);
     for (cudaEvent_t &e : done_) {
-      if (!e) continue;
-      cudaEventSynchronize(e);
-      cudaEventDestroy(e);
+      if (e) cudaEventDestroy(e);
       e = nullptr;
     }
+    if (order_) cudaEventDestroy(order_);
+    order_ = nullptr;
+    if (stream_) cudaStreamDestroy(stream_);
+    stream_ = nullptr;
     if (memory_) cudaFreeHost(memory_);
     memory_ = nullptr;
   }
 
  private:
+  static bool pageable(const void *p) {
+    cudaPointerAttributes attr;
+    return cudaPointerGetAttributes(&attr, p) == cudaSuccess &&
+           attr.type == cudaMemoryTypeUnregistered;
+  }
+  static bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus status;
+    return cudaStreamIsCapturing(s, &status) != cudaSuccess ||
+           status != cudaStreamCaptureStatusNone;
+  }
+  // what is queued on `later` from here on starts after `earlier`'s work
+  cudaError_t follow(cudaStream_t later, cudaStream_t earlier) {
+    const cudaError_t r = cudaEventRecord(order_, earlier);
+    return r != cudaSuccess ? r : cudaStreamWaitEvent(later, order_, 0);
+  }
   bool make() {
     if (memory_) return true;
     for (cudaEvent_t &e : done_)
       if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return false;
+    if (!order_ && cudaEventCreateWithFlags(&order_, cudaEventDisableTiming) != cudaSuccess)
+      return false;
+    if (!stream_ && cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking) != cudaSuccess)
+      return false;
     return cudaHostAlloc((void **)&memory_, 2 * kThreads * kPiece, cudaHostAllocDefault) ==
            cudaSuccess;
   }
   uint8_t *memory_ = nullptr;
+  cudaStream_t stream_ = nullptr;
+  cudaEvent_t order_ = nullptr;
   cudaEvent_t done_[2 * kThreads] = {};
 };
 

@@ -43,3 +43,37 @@ def test_pageable_and_pinned_uploads(length):
                                       number_sequences=len(offsets) - 1))
     finally:
         e.close()
+
+
+def test_per_thread_default_stream():
+    """The per-thread default stream's handle means another stream in every
+    thread: the staged pieces have to arrive between the work queued before
+    and after the upload on the calling thread's."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from gzb import native as N
+    per_thread = 2  # cudaStreamPerThread
+    length = 48 << 20
+    rng = np.random.default_rng(5)
+    offsets = np.arange(1, length - 300, 300, dtype=np.uint32)
+    chunks = []
+    for _ in range(2):
+        codes = rng.integers(0, 20, length).astype(np.uint8)
+        codes[offsets - 1] = P.DELIMITER
+        codes[-1] = P.DELIMITER
+        chunks.append(codes)
+    offs = np.append(offsets, length).astype(np.uint32)
+    e = N.PresearchEngine(0)
+    try:
+        e.set_params(P.make_params())
+
+        def index(codes, **stream):
+            db = W.Database(codes=codes, offsets=offs, number_sequences=len(offs) - 1)
+            e.set_database(db, **stream)
+            return e.export_index(**stream)
+        want = [index(torch.from_numpy(c).pin_memory().numpy()) for c in chunks]
+        for k in (0, 1, 0, 1, 1, 0):
+            assert np.array_equal(index(chunks[k], stream=per_thread), want[k])
+    finally:
+        e.close()
