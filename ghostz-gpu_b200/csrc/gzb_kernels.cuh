@@ -190,8 +190,12 @@ __device__ __forceinline__ void load_walk_words(WalkWords<INC> &ww, const uint8_
 // against stop_above, once at its end.  A chunk in which the walk ends is
 // then replayed pair by pair from its start (the exact exit pair, its best
 // and the step count); no pair after a delimiter changes a value the walk
-// returns, since the delimiter's -32768 ends the replay first.
-template <int INC>
+// returns, since the delimiter's -32768 ends the replay first.  kCodes: the
+// bits of a byte that are a residue code; where the bytes behind a delimiter
+// may be anything (the operators' buffers), only those index the table.
+constexpr uint32_t kAnyByte = 0xffffffffu, kCodeBits = 0x1f1f1f1fu;
+
+template <int INC, uint32_t kCodes = kAnyByte>
 __device__ __forceinline__ int walk_side_words(const WalkWords<INC> &A, const WalkWords<INC> &B,
                                                const char *tbl, int cutoff, int stop_above,
                                                int *steps, int score, int best) {
@@ -223,11 +227,11 @@ __device__ __forceinline__ int walk_side_words(const WalkWords<INC> &A, const Wa
   }
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    const uint32_t qa = INC > 0 ? __funnelshift_r(A.w[k], A.w[k + 1], sha)
-                                : __funnelshift_r(A.w[k + 1], A.w[k], sha);
+    const uint32_t qa = (INC > 0 ? __funnelshift_r(A.w[k], A.w[k + 1], sha)
+                                 : __funnelshift_r(A.w[k + 1], A.w[k], sha)) & kCodes;
     const uint32_t qb = INC > 0 ? __funnelshift_r(B.w[k], B.w[k + 1], shb)
                                 : __funnelshift_r(B.w[k + 1], B.w[k], shb);
-    const uint32_t x4p = (qa ^ qb) << 2;
+    const uint32_t x4p = ((qa ^ qb) & kCodes) << 2;
     GZB_WALK_CHUNK(x4p, qa)
   }
   {
@@ -250,8 +254,8 @@ __device__ __forceinline__ int walk_side_words(const WalkWords<INC> &A, const Wa
       b_lo = __ldg(pb);
     }
     for (;;) {
-      const uint32_t qa = __funnelshift_r(a_lo, a_hi, sha);
-      const uint32_t x4 = (qa ^ __funnelshift_r(b_lo, b_hi, shb)) << 2;
+      const uint32_t qa = __funnelshift_r(a_lo, a_hi, sha) & kCodes;
+      const uint32_t x4 = ((qa ^ __funnelshift_r(b_lo, b_hi, shb)) & kCodes) << 2;
       GZB_WALK_CHUNK(x4, qa)
       if (INC > 0) {
         a_lo = a_hi;
@@ -299,20 +303,21 @@ done:
 // from s0[0]/s1[0] (query/database) stepping by INC: returns the best prefix
 // score, stopping at the X-drop (best - score >= cutoff, cutoff >= 1), at a
 // delimiter, or once the best exceeds stop_above.  The reference's
-// (best, run) pair is (best, score - best) here; a walk may go on from one.  Reads four residue pairs
-// per pair of aligned 32-bit words.  The first kWalkPrefetch chunks' words
-// are loaded together up front (most walks end inside them, so a walk waits
-// for one round of loads instead of one per chunk); a longer walk goes on
-// one word per chunk.  The sequences carry delimiter padding of at least
-// 4 (kWalkPrefetch + 1) bytes on each side.  *steps counts pairs examined.
-template <int INC>
+// (best, run) pair is (best, score - best) here; a walk may go on from one.
+// Reads four residue pairs per pair of aligned 32-bit words.  The first
+// kWalkPrefetch chunks' words are loaded together up front (most walks end
+// inside them, so a walk waits for one round of loads instead of one per
+// chunk); a longer walk goes on one word per chunk.  At least
+// 4 (kWalkPrefetch + 1) bytes are readable on each side of the sequences.
+// *steps counts pairs examined.
+template <int INC, uint32_t kCodes = kAnyByte>
 __device__ __forceinline__ int walk_side(const uint8_t *s0, const uint8_t *s1,
                                          const char *tbl, int cutoff, int stop_above,
                                          int *steps, int score = 0, int best = 0) {
   WalkWords<INC> A, B;
   load_walk_words(A, s0);
   load_walk_words(B, s1);
-  return walk_side_words(A, B, tbl, cutoff, stop_above, steps, score, best);
+  return walk_side_words<INC, kCodes>(A, B, tbl, cutoff, stop_above, steps, score, best);
 }
 
 // Whether the X-drop walk from s0[0]/s1[0] stepping by INC survives its
@@ -382,11 +387,12 @@ __device__ __forceinline__ bool walk_reaches(const uint8_t *s0, const uint8_t *s
 // SeedSearcher::UngappedExtend on the walk table: reverse from (q-1, d-1),
 // forward from (q, d) unless the reverse best already exceeds trigger; true
 // when the sum exceeds trigger.
+template <uint32_t kCodes = kAnyByte>
 __device__ __forceinline__ bool walk_hit(const uint8_t *q, const uint8_t *d, const char *tbl,
                                          int cutoff, int trigger, int *steps) {
-  int sum = walk_side<-1>(q - 1, d - 1, tbl, cutoff, trigger, steps);
+  int sum = walk_side<-1, kCodes>(q - 1, d - 1, tbl, cutoff, trigger, steps);
   if (sum > trigger) return true;
-  sum += walk_side<1>(q, d, tbl, cutoff, trigger - sum, steps);
+  sum += walk_side<1, kCodes>(q, d, tbl, cutoff, trigger - sum, steps);
   return sum > trigger;
 }
 

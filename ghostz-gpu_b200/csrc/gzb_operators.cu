@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kUngappedBlock, 3) ungapped_trigger_kernel(
       const uint8_t *qs = q + qpos[i], *ds = d + dpos[i];
       int steps = 0;
       flags[i] = coded && cutoff >= 1 && cutoff <= kWalkMaxDrop
-                     ? walk_hit(qs, ds, walk, cutoff, trigger, &steps)
+                     ? walk_hit<kCodeBits>(qs, ds, walk, cutoff, trigger, &steps)
                      : ungapped_hit(qs, ds, delim, sh.matrix, cutoff, trigger, &steps);
     }
   };

@@ -127,7 +127,8 @@ __host__ __device__ __forceinline__ uint32_t window_addmax(uint32_t a, uint32_t 
 #endif
 }
 
-// Both walks over the window.  bests: the sum of the two sides' largest
+// Both walks over the window; a byte of q or d of 32 or more is no table
+// address.  bests: the sum of the two sides' largest
 // (doubled) scores, from after a walk's end too unless kExact, where a score
 // falls by 256 a step from there on and so stays below its best.  steps and
 // delimiters (per half): the steps from the end on, and of those the ones
@@ -232,11 +233,18 @@ __device__ __forceinline__ bool walk_on(const uint8_t *q, const uint8_t *d, cons
 #endif
 
 // 1: a hit (scores the walks reach sum to more than the trigger), 0: none
-// (both walks end), -1: open.
+// (both walks end), -1: open.  The bytes behind a delimiter may be anything:
+// their low five bits stand in, which no score or flag depends on.
 __host__ __device__ __forceinline__ int walk_window_hit(uint32_t tbl, const uint32_t q[16],
                                                         const uint32_t d[16], int cutoff,
                                                         int trigger) {
-  const WindowWalk w = walk_both<true>(tbl, q, d, cutoff);
+  uint32_t qc[16], dc[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    qc[i] = q[i] & kCodeBits;
+    dc[i] = d[i] & kCodeBits;
+  }
+  const WindowWalk w = walk_both<true>(tbl, qc, dc, cutoff);
   return w.bests > 2 * trigger ? 1 : w.steps[0] > 0 && w.steps[1] > 0 ? 0 : -1;
 }
 

@@ -77,7 +77,9 @@ typedef struct {
 /* Device sequence buffers given to the operators below hold one residue
  * code (< 32) per byte, sequences separated by the delimiter, with at least
  * 64 delimiter bytes before the first and after the last sequence: the
- * kernels read aligned 32-bit words, a few bytes past a delimiter. */
+ * kernels read aligned words, up to 63 bytes either side of a seed whatever
+ * delimiters lie between.  No extension depends on what stands behind the
+ * first delimiter either side of its seed. */
 
 /* ---- DistanceCalculatorGpu (src/distance_calculator_gpu.h:18-40) ------- */
 typedef struct gzb_distance_calculator gzb_distance_calculator;
