@@ -100,8 +100,8 @@ __global__ void distance_kernel(const uint8_t *__restrict__ q,
 // Ungapped extension with trigger.  A seed's window of 32 residues either
 // side is evaluated first (gzb_walk.cuh: no branches, three loads a
 // sequence); the seeds that leaves open wait until a warp has 32 to walk.
-// The tables hold delimiters and cutoffs in a code's and a word's half's
-// range, others are walked pair by pair (kWalkMaxDrop: what a delimiter's
+// A delimiter is a code of the tables (below 32); cutoffs outside a word's
+// half's range are walked pair by pair (kWalkMaxDrop: what a delimiter's
 // entry of the walk table still ends).
 // 3,000,000 seeds of 2,048 queries: 306 us with a walk a thread, this
 // 195 (50,000 seeds: 20.6 and 13.5); of these seeds 85 in 100 are hits, nearly
@@ -126,11 +126,10 @@ __global__ void __launch_bounds__(kUngappedBlock, 3) ungapped_trigger_kernel(
   __shared__ UngappedShared sh;
   load_matrix(sh.matrix, matrix, number_letters, stride);
   __syncthreads();
-  const bool coded = delim < 32;
   const uint32_t window = (uint32_t)__cvta_generic_to_shared(sh.window);
   const char *walk = reinterpret_cast<const char *>(sh.walk);
   load_walk_table(sh.walk, sh.matrix, delim, kMatrixStride);
-  const bool fits = load_window_table(window, sh.matrix, delim, kMatrixStride) && coded;
+  const bool fits = load_window_table(window, sh.matrix, delim, kMatrixStride);
   WarpStack<uint64_t> open;
   open.item = sh.open[threadIdx.x >> 5];
   auto run_open = [&]() {
@@ -140,7 +139,7 @@ __global__ void __launch_bounds__(kUngappedBlock, 3) ungapped_trigger_kernel(
       const int cutoff = cutoffs[id], trigger = triggers[id];
       const uint8_t *qs = q + qpos[i], *ds = d + dpos[i];
       int steps = 0;
-      flags[i] = coded && cutoff >= 1 && cutoff <= kWalkMaxDrop
+      flags[i] = cutoff >= 1 && cutoff <= kWalkMaxDrop
                      ? walk_hit<kCodeBits>(qs, ds, walk, cutoff, trigger, &steps)
                      : ungapped_hit(qs, ds, delim, sh.matrix, cutoff, trigger, &steps);
     }
@@ -171,6 +170,29 @@ __global__ void __launch_bounds__(kUngappedBlock, 3) ungapped_trigger_kernel(
     if (open.n >= 32) run_open();
   }
   while (open.n) run_open();
+}
+
+// The same for a delimiter that is no code (32 and more), a seed a thread,
+// pair by pair: 1,000,000 seeds 117 us; through the stack of
+// ungapped_trigger_kernel, at its three blocks an SM, 143.
+__global__ void ungapped_pairs_kernel(
+    const uint8_t *__restrict__ q, const uint8_t *__restrict__ d, int delim,
+    const int32_t *__restrict__ matrix, int number_letters, int stride,
+    const int32_t *__restrict__ cutoffs, const int32_t *__restrict__ triggers,
+    size_t n, const uint32_t *__restrict__ qid,
+    const uint32_t *__restrict__ qpos, const uint32_t *__restrict__ dpos,
+    int8_t *__restrict__ flags) {
+  __shared__ int sm[kMatrixStride * kMatrixStride];
+  load_matrix(sm, matrix, number_letters, stride);
+  __syncthreads();
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const uint32_t id = qid[i];
+    int steps = 0;
+    flags[i] = ungapped_hit(q + qpos[i], d + dpos[i], delim, sm, cutoffs[id], triggers[id], &steps)
+                   ? 1
+                   : 0;
+  }
 }
 
 // set[start[i]] = i (the run-start scatter of SetQuerySeeds).
@@ -1075,7 +1097,9 @@ extern "C" int gzb_ungapped_extender_extend_with_trigger_async(
   if (qid) GZB_CUDA(cudaMemcpyAsync(d_qid, qid, 4 * size, cudaMemcpyDefault, s));
   if (qpos) GZB_CUDA(cudaMemcpyAsync(d_qpos, qpos, 4 * size, cudaMemcpyDefault, s));
   if (dpos) GZB_CUDA(cudaMemcpyAsync(d_dpos, dpos, 4 * size, cudaMemcpyDefault, s));
-  ungapped_trigger_kernel<<<grid_for(size, kUngappedBlock, 148 * 3), kUngappedBlock, 0, s>>>(
+  const bool coded = h->delim < 32;
+  auto kernel = coded ? ungapped_trigger_kernel : ungapped_pairs_kernel;
+  kernel<<<grid_for(size, kUngappedBlock, 148 * (coded ? 3 : 16)), kUngappedBlock, 0, s>>>(
       h->queries, h->db, h->delim, h->matrix, (int)h->number_letters,
       (int)h->number_letters + 1, h->cutoffs, h->triggers, size, d_qid, d_qpos, d_dpos,
       d_flags);
