@@ -282,9 +282,9 @@ __device__ __forceinline__ void store_result(uint32_t e, uint32_t q, uint32_t d,
 }
 
 // One extension on one thread, a database row at a time.  FAST: the grouped
-// rows of gzb_row.cuh, for the parameters row_dp_exact admits (three quarters
-// of the other form's time, see there); else lane_init / lane_row, for every
-// X-drop.
+// rows of gzb_row.cuh, for the parameters row_dp_exact and the matrix entries
+// row_entry_fits admit (three quarters of the other form's time, see there);
+// else lane_init / lane_row, for every X-drop and matrix.
 __host__ __device__ constexpr int lane_table_words(bool fast) {
   return fast ? kRowTableWords : kMatrixStride * kMatrixStride;
 }
@@ -322,7 +322,7 @@ struct LaneWork<W, true> {
   uint32_t tbl;  // shared-memory address
   RowBand<W, kLaneBlock> band;
   RowExt x;
-  bool fits;  // the matrix (a larger one hands every extension on)
+  bool fits;  // the matrix
   __device__ __forceinline__ LaneWork(const GappedJob &job, int *tbl_, uint32_t *cells,
                                       uint8_t *res, const int32_t *matrix, int number_letters,
                                       int stride)
@@ -332,8 +332,7 @@ struct LaneWork<W, true> {
     fits = load_row_table(tbl_, job, matrix, number_letters, stride);
   }
   __device__ __forceinline__ int init(const GappedJob &job, uint32_t q, uint32_t d, bool rev) {
-    const int st = row_init<W, kLaneBlock>(job, band, x, job.query + q, job.db + d, rev);
-    return fits ? st : kLaneOverflow;
+    return row_init<W, kLaneBlock>(job, band, x, job.query + q, job.db + d, rev);
   }
   __device__ __forceinline__ int step(const GappedJob &job, int st) {
     return row_step<W, kLaneBlock>(job, tbl, band, x, st);
@@ -343,6 +342,25 @@ struct LaneWork<W, true> {
   __device__ __forceinline__ int pos0() const { return x.pos0(); }
   __device__ __forceinline__ int pos1() const { return x.pos1(); }
 };
+
+// run(the extension state of this thread).  The matrix may be known to the
+// device alone, so a FAST kernel holds the other form, too: 600,000
+// extensions with -2000 for the stop letter 11.4 ms, handed on to the warp
+// kernel 17.4.
+template <int W, bool FAST, class Run>
+__device__ __forceinline__ void with_lane_work(const GappedJob &job, int *tbl, uint32_t *cells,
+                                               uint8_t *res, const int32_t *matrix,
+                                               int number_letters, int stride, Run run) {
+  if constexpr (FAST) {
+    LaneWork<W, true> x(job, tbl, cells, res, matrix, number_letters, stride);
+    if (x.fits) {
+      run(x);
+      return;
+    }
+  }
+  LaneWork<W, false> x(job, tbl, cells, res, matrix, number_letters, stride);
+  run(x);
+}
 
 template <bool FAST>
 __global__ void __launch_bounds__(kLaneBlock)
@@ -355,40 +373,42 @@ gapped_lane_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
   __shared__ __align__(16) uint32_t cells_s[kLaneW * kLaneBlock];
   __shared__ __align__(4) uint8_t res_s[kLaneW * kLaneBlock];
   if (n_dev) n = *n_dev;
-  LaneWork<kLaneW, FAST> x(job, sm, cells_s, res_s, matrix, number_letters, stride);
-  unsigned long long cells = 0;
-  const size_t lane = threadIdx.x & 31;
-  for (size_t i0 = blockIdx.x * (size_t)blockDim.x + (threadIdx.x & ~31u); i0 < n;
-       i0 += (size_t)gridDim.x * blockDim.x) {
-    const size_t i = i0 + lane;
-    uint32_t e = 0, q = 0, d = 0;
-    int st = kLaneDone;
-    if (i < n) {
-      e = order ? order[i] : (uint32_t)i;
-      const bool rev = dir ? dir[e] != 0 : reverse != 0;
-      q = qpos[e];
-      d = dpos[e];
-      st = x.init(job, q, d, rev);
+  auto run = [&](auto &x) {
+    unsigned long long cells = 0;
+    const size_t lane = threadIdx.x & 31;
+    for (size_t i0 = blockIdx.x * (size_t)blockDim.x + (threadIdx.x & ~31u); i0 < n;
+         i0 += (size_t)gridDim.x * blockDim.x) {
+      const size_t i = i0 + lane;
+      uint32_t e = 0, q = 0, d = 0;
+      int st = kLaneDone;
+      if (i < n) {
+        e = order ? order[i] : (uint32_t)i;
+        const bool rev = dir ? dir[e] != 0 : reverse != 0;
+        q = qpos[e];
+        d = dpos[e];
+        st = x.init(job, q, d, rev);
+      }
+      while (__any_sync(0xffffffffu, st == kLaneRunning)) st = x.step(job, st);
+      if (i >= n) {
+      } else if (x.overflow(st)) {
+        spill[atomicAdd(spill_count, 1u)] = e;
+        if (cells_out) cells_out[e] = 0xFFFFFFFFu;
+      } else {
+        cells += x.x.cells;
+        qpos[e] = q + (uint32_t)x.pos0();
+        dpos[e] = d + (uint32_t)x.pos1();
+        scores[e] = x.score();
+        if (cells_out) cells_out[e] = x.x.cells;
+      }
     }
-    while (__any_sync(0xffffffffu, st == kLaneRunning)) st = x.step(job, st);
-    if (i >= n) {
-    } else if (x.overflow(st)) {
-      spill[atomicAdd(spill_count, 1u)] = e;
-      if (cells_out) cells_out[e] = 0xFFFFFFFFu;
-    } else {
-      cells += x.x.cells;
-      qpos[e] = q + (uint32_t)x.pos0();
-      dpos[e] = d + (uint32_t)x.pos1();
-      scores[e] = x.score();
-      if (cells_out) cells_out[e] = x.x.cells;
-    }
-  }
-  cells += __shfl_down_sync(0xffffffffu, cells, 16);
-  cells += __shfl_down_sync(0xffffffffu, cells, 8);
-  cells += __shfl_down_sync(0xffffffffu, cells, 4);
-  cells += __shfl_down_sync(0xffffffffu, cells, 2);
-  cells += __shfl_down_sync(0xffffffffu, cells, 1);
-  if ((threadIdx.x & 31) == 0 && cells) atomicAdd(cells_total, cells);
+    cells += __shfl_down_sync(0xffffffffu, cells, 16);
+    cells += __shfl_down_sync(0xffffffffu, cells, 8);
+    cells += __shfl_down_sync(0xffffffffu, cells, 4);
+    cells += __shfl_down_sync(0xffffffffu, cells, 2);
+    cells += __shfl_down_sync(0xffffffffu, cells, 1);
+    if ((threadIdx.x & 31) == 0 && cells) atomicAdd(cells_total, cells);
+  };
+  with_lane_work<kLaneW, FAST>(job, sm, cells_s, res_s, matrix, number_letters, stride, run);
 }
 
 // Flattened one-thread-per-extension kernel over a device work queue
@@ -430,45 +450,47 @@ gapped_lane_queue_kernel(GappedJob job, const int32_t *__restrict__ matrix, int 
   __shared__ __align__(16) uint32_t cells_s[kLaneW * kLaneBlock];
   __shared__ __align__(4) uint8_t res_s[kLaneW * kLaneBlock];
   if (n_dev) n = *n_dev;
-  LaneWork<kLaneW, FAST> x(job, sm, cells_s, res_s, matrix, number_letters, stride);
-  const int lane = threadIdx.x & 31;
-  unsigned long long cells = 0;
-  for (;;) {
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(queue, 32ull);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= n) break;
-    const uint64_t i = base + lane;
-    uint32_t e = 0, q = 0, d = 0;
-    int st = kLaneDone;
-    if (i < n) {
-      e = order ? order[i] : (uint32_t)i;
-      const bool rev = dir ? dir[e] != 0 : reverse != 0;
-      q = qpos[e];
-      d = dpos[e];
-      st = x.init(job, q, d, rev);
-    }
-    while (__any_sync(0xffffffffu, st == kLaneRunning)) st = x.step(job, st);
-    if (i < n) {
-      if (x.overflow(st)) {
-        spill[atomicAdd(spill_count, 1u)] = e;
-        if (cells_out) cells_out[e] = 0xFFFFFFFFu;
-      } else {
-        cells += x.x.cells;
-        qpos[e] = q + (uint32_t)x.pos0();
-        dpos[e] = d + (uint32_t)x.pos1();
-        scores[e] = x.score();
-        if (cells_out) cells_out[e] = x.x.cells;
+  auto run = [&](auto &x) {
+    const int lane = threadIdx.x & 31;
+    unsigned long long cells = 0;
+    for (;;) {
+      unsigned long long base = 0;
+      if (lane == 0) base = atomicAdd(queue, 32ull);
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (base >= n) break;
+      const uint64_t i = base + lane;
+      uint32_t e = 0, q = 0, d = 0;
+      int st = kLaneDone;
+      if (i < n) {
+        e = order ? order[i] : (uint32_t)i;
+        const bool rev = dir ? dir[e] != 0 : reverse != 0;
+        q = qpos[e];
+        d = dpos[e];
+        st = x.init(job, q, d, rev);
       }
+      while (__any_sync(0xffffffffu, st == kLaneRunning)) st = x.step(job, st);
+      if (i < n) {
+        if (x.overflow(st)) {
+          spill[atomicAdd(spill_count, 1u)] = e;
+          if (cells_out) cells_out[e] = 0xFFFFFFFFu;
+        } else {
+          cells += x.x.cells;
+          qpos[e] = q + (uint32_t)x.pos0();
+          dpos[e] = d + (uint32_t)x.pos1();
+          scores[e] = x.score();
+          if (cells_out) cells_out[e] = x.x.cells;
+        }
+      }
+      __syncwarp();
     }
-    __syncwarp();
-  }
-  cells += __shfl_down_sync(0xffffffffu, cells, 16);
-  cells += __shfl_down_sync(0xffffffffu, cells, 8);
-  cells += __shfl_down_sync(0xffffffffu, cells, 4);
-  cells += __shfl_down_sync(0xffffffffu, cells, 2);
-  cells += __shfl_down_sync(0xffffffffu, cells, 1);
-  if (lane == 0 && cells) atomicAdd(cells_total, cells);
+    cells += __shfl_down_sync(0xffffffffu, cells, 16);
+    cells += __shfl_down_sync(0xffffffffu, cells, 8);
+    cells += __shfl_down_sync(0xffffffffu, cells, 4);
+    cells += __shfl_down_sync(0xffffffffu, cells, 2);
+    cells += __shfl_down_sync(0xffffffffu, cells, 1);
+    if (lane == 0 && cells) atomicAdd(cells_total, cells);
+  };
+  with_lane_work<kLaneW, FAST>(job, sm, cells_s, res_s, matrix, number_letters, stride, run);
 }
 
 // Row-granular work queue: every lane runs its own extension one database
@@ -506,49 +528,51 @@ gapped_rows_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
   uint32_t *cells_s = kStatic ? cells_st : reinterpret_cast<uint32_t *>(rows_band);
   uint8_t *res_s = kStatic ? res_st : rows_band + (size_t)W * kLaneBlock * 4;
   if (n_dev) n = *n_dev;
-  LaneWork<W, FAST> x(job, sm, cells_s, res_s, matrix, number_letters, stride);
-  uint32_t e = 0, q = 0, d = 0;
-  bool have = false, done = false;
-  unsigned long long cells = 0;
-  for (;;) {
-    int st = x.step(job, have ? kLaneRunning : kLaneDone);
-    const unsigned idle = __ballot_sync(0xffffffffu, !done && (!have || st != kLaneRunning));
-    const unsigned busy = __ballot_sync(0xffffffffu, have && st == kLaneRunning);
-    if (idle == 0 && busy == 0) break;
-    const bool refill = __popc(idle) >= refill_threshold || busy == 0;
-    while (have ? st != kLaneRunning : (refill && !done)) {
-      if (have) {  // the extension ended: write it out
-        if (x.overflow(st)) {
-          spill[atomicAdd(spill_count, 1u)] = e;
-          if (cells_out) cells_out[e] = 0xFFFFFFFFu;
-        } else {
-          cells += x.x.cells;
-          qpos[e] = q + (uint32_t)x.pos0();
-          dpos[e] = d + (uint32_t)x.pos1();
-          scores[e] = x.score();
-          if (cells_out) cells_out[e] = x.x.cells;
+  auto run = [&](auto &x) {
+    uint32_t e = 0, q = 0, d = 0;
+    bool have = false, done = false;
+    unsigned long long cells = 0;
+    for (;;) {
+      int st = x.step(job, have ? kLaneRunning : kLaneDone);
+      const unsigned idle = __ballot_sync(0xffffffffu, !done && (!have || st != kLaneRunning));
+      const unsigned busy = __ballot_sync(0xffffffffu, have && st == kLaneRunning);
+      if (idle == 0 && busy == 0) break;
+      const bool refill = __popc(idle) >= refill_threshold || busy == 0;
+      while (have ? st != kLaneRunning : (refill && !done)) {
+        if (have) {  // the extension ended: write it out
+          if (x.overflow(st)) {
+            spill[atomicAdd(spill_count, 1u)] = e;
+            if (cells_out) cells_out[e] = 0xFFFFFFFFu;
+          } else {
+            cells += x.x.cells;
+            qpos[e] = q + (uint32_t)x.pos0();
+            dpos[e] = d + (uint32_t)x.pos1();
+            scores[e] = x.score();
+            if (cells_out) cells_out[e] = x.x.cells;
+          }
+          have = false;
+          st = kLaneRunning;
+          if (!refill) break;
         }
-        have = false;
-        st = kLaneRunning;
-        if (!refill) break;
+        if (!flat_fetch(queue, n, order, &e)) {
+          done = true;
+          break;
+        }
+        const bool rev = dir ? dir[e] != 0 : reverse != 0;
+        q = qpos[e];
+        d = dpos[e];
+        st = x.init(job, q, d, rev);
+        have = true;
       }
-      if (!flat_fetch(queue, n, order, &e)) {
-        done = true;
-        break;
-      }
-      const bool rev = dir ? dir[e] != 0 : reverse != 0;
-      q = qpos[e];
-      d = dpos[e];
-      st = x.init(job, q, d, rev);
-      have = true;
     }
-  }
-  cells += __shfl_down_sync(0xffffffffu, cells, 16);
-  cells += __shfl_down_sync(0xffffffffu, cells, 8);
-  cells += __shfl_down_sync(0xffffffffu, cells, 4);
-  cells += __shfl_down_sync(0xffffffffu, cells, 2);
-  cells += __shfl_down_sync(0xffffffffu, cells, 1);
-  if ((threadIdx.x & 31) == 0 && cells) atomicAdd(cells_total, cells);
+    cells += __shfl_down_sync(0xffffffffu, cells, 16);
+    cells += __shfl_down_sync(0xffffffffu, cells, 8);
+    cells += __shfl_down_sync(0xffffffffu, cells, 4);
+    cells += __shfl_down_sync(0xffffffffu, cells, 2);
+    cells += __shfl_down_sync(0xffffffffu, cells, 1);
+    if ((threadIdx.x & 31) == 0 && cells) atomicAdd(cells_total, cells);
+  };
+  with_lane_work<W, FAST>(job, sm, cells_s, res_s, matrix, number_letters, stride, run);
 }
 
 // Row-step refill with extensions dealt round-robin: lane t of the grid
@@ -566,59 +590,61 @@ gapped_deal_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
   __shared__ __align__(16) uint32_t cells_s[kLaneW * kLaneBlock];
   __shared__ __align__(4) uint8_t res_s[kLaneW * kLaneBlock];
   if (n_dev) n = *n_dev;
-  LaneWork<kLaneW, FAST> x(job, sm, cells_s, res_s, matrix, number_letters, stride);
-  const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
-  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  // the next extension of this lane, loaded one extension ahead
-  uint32_t ne = 0, nq = 0, nd = 0;
-  bool nrev = false;
-  auto load_next = [&](uint64_t k) {
-    if (k < n) {
-      ne = order ? order[k] : (uint32_t)k;
-      nq = qpos[ne];
-      nd = dpos[ne];
-      nrev = dir ? dir[ne] != 0 : reverse != 0;
-    }
-  };
-  load_next(i);
-  uint32_t e = 0, q = 0, d = 0;
-  bool have = false;
-  unsigned long long cells = 0;
-  for (;;) {
-    int st = x.step(job, have ? kLaneRunning : kLaneDone);
-    if (!have) st = kLaneRunning;
-    while (st != kLaneRunning || (!have && i < n)) {
-      if (have) {  // the extension ended: write it out
-        if (x.overflow(st)) {
-          spill[atomicAdd(spill_count, 1u)] = e;
-          if (cells_out) cells_out[e] = 0xFFFFFFFFu;
-        } else {
-          cells += x.x.cells;
-          qpos[e] = q + (uint32_t)x.pos0();
-          dpos[e] = d + (uint32_t)x.pos1();
-          scores[e] = x.score();
-          if (cells_out) cells_out[e] = x.x.cells;
-        }
-        have = false;
-        i += T;
+  auto run = [&](auto &x) {
+    const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
+    uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    // the next extension of this lane, loaded one extension ahead
+    uint32_t ne = 0, nq = 0, nd = 0;
+    bool nrev = false;
+    auto load_next = [&](uint64_t k) {
+      if (k < n) {
+        ne = order ? order[k] : (uint32_t)k;
+        nq = qpos[ne];
+        nd = dpos[ne];
+        nrev = dir ? dir[ne] != 0 : reverse != 0;
       }
-      if (i >= n) break;
-      e = ne;
-      q = nq;
-      d = nd;
-      const bool rev = nrev;
-      load_next(i + T);
-      st = x.init(job, q, d, rev);
-      have = true;
+    };
+    load_next(i);
+    uint32_t e = 0, q = 0, d = 0;
+    bool have = false;
+    unsigned long long cells = 0;
+    for (;;) {
+      int st = x.step(job, have ? kLaneRunning : kLaneDone);
+      if (!have) st = kLaneRunning;
+      while (st != kLaneRunning || (!have && i < n)) {
+        if (have) {  // the extension ended: write it out
+          if (x.overflow(st)) {
+            spill[atomicAdd(spill_count, 1u)] = e;
+            if (cells_out) cells_out[e] = 0xFFFFFFFFu;
+          } else {
+            cells += x.x.cells;
+            qpos[e] = q + (uint32_t)x.pos0();
+            dpos[e] = d + (uint32_t)x.pos1();
+            scores[e] = x.score();
+            if (cells_out) cells_out[e] = x.x.cells;
+          }
+          have = false;
+          i += T;
+        }
+        if (i >= n) break;
+        e = ne;
+        q = nq;
+        d = nd;
+        const bool rev = nrev;
+        load_next(i + T);
+        st = x.init(job, q, d, rev);
+        have = true;
+      }
+      if (!__any_sync(0xffffffffu, have)) break;
     }
-    if (!__any_sync(0xffffffffu, have)) break;
-  }
-  cells += __shfl_down_sync(0xffffffffu, cells, 16);
-  cells += __shfl_down_sync(0xffffffffu, cells, 8);
-  cells += __shfl_down_sync(0xffffffffu, cells, 4);
-  cells += __shfl_down_sync(0xffffffffu, cells, 2);
-  cells += __shfl_down_sync(0xffffffffu, cells, 1);
-  if ((threadIdx.x & 31) == 0 && cells) atomicAdd(cells_total, cells);
+    cells += __shfl_down_sync(0xffffffffu, cells, 16);
+    cells += __shfl_down_sync(0xffffffffu, cells, 8);
+    cells += __shfl_down_sync(0xffffffffu, cells, 4);
+    cells += __shfl_down_sync(0xffffffffu, cells, 2);
+    cells += __shfl_down_sync(0xffffffffu, cells, 1);
+    if ((threadIdx.x & 31) == 0 && cells) atomicAdd(cells_total, cells);
+  };
+  with_lane_work<kLaneW, FAST>(job, sm, cells_s, res_s, matrix, number_letters, stride, run);
 }
 
 // process-wide tile defaults (gzb_set_tile_parameter)
