@@ -282,9 +282,9 @@ __device__ __forceinline__ void store_result(uint32_t e, uint32_t q, uint32_t d,
 }
 
 // One extension on one thread, a database row at a time.  FAST: the grouped
-// rows of gzb_row.cuh, for the parameters row_dp_exact and the matrix entries
-// row_entry_fits admit (three quarters of the other form's time, see there);
-// else lane_init / lane_row, for every X-drop and matrix.
+// rows of gzb_row.cuh, for the parameters row_dp_exact and row_dp_pays and the
+// matrix entries row_entry_fits admit (three quarters of the other form's
+// time, see there); else lane_init / lane_row, for every X-drop and matrix.
 __host__ __device__ constexpr int lane_table_words(bool fast) {
   return fast ? kRowTableWords : kMatrixStride * kMatrixStride;
 }
@@ -751,9 +751,14 @@ static int launch_gapped_rows_as(const GappedTile &tile, const GappedJob &job,
   return GZB_OK;
 }
 
+static bool grouped_rows(const GappedJob &job) {
+  return row_dp_exact(job.gap_open, job.gap_ext, job.cutoff) &&
+         row_dp_pays(job.gap_open, job.gap_ext, job.cutoff);
+}
+
 template <int W, typename... Args>
 static int launch_gapped_rows(const GappedTile &tile, const GappedJob &job, Args... args) {
-  return row_dp_exact(job.gap_open, job.gap_ext, job.cutoff)
+  return grouped_rows(job)
              ? launch_gapped_rows_as<W, true>(tile, job, args...)
              : launch_gapped_rows_as<W, false>(tile, job, args...);
 }
@@ -765,7 +770,7 @@ int launch_gapped_static(unsigned blocks, const GappedJob &job, const int32_t *m
                          int32_t *scores, uint32_t *spill, uint32_t *spill_count,
                          unsigned long long *cells_total, uint32_t *cells_out, cudaStream_t s,
                          const uint64_t *n_dev) {
-  auto kernel = row_dp_exact(job.gap_open, job.gap_ext, job.cutoff) ? gapped_lane_kernel<true>
+  auto kernel = grouped_rows(job) ? gapped_lane_kernel<true>
                                                                     : gapped_lane_kernel<false>;
   kernel<<<blocks, kLaneBlock, 0, s>>>(job, matrix, number_letters, stride, n, order, reverse,
                                        dir, qpos, dpos, scores, spill, spill_count, cells_total,
@@ -784,7 +789,7 @@ int launch_gapped_thread(const GappedTile &tile, const GappedJob &job, const int
   // (grids sized for n)
   GZB_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s));
   uint64_t blocks = 1;
-  const bool fast = row_dp_exact(job.gap_open, job.gap_ext, job.cutoff);
+  const bool fast = grouped_rows(job);
   const bool group = tile.kernel >= GZB_GAPPED_KERNEL_GROUP4 &&
                      tile.kernel <= GZB_GAPPED_KERNEL_GROUP32 && warp_path_exact(job.cutoff);
   if (group) {

@@ -224,6 +224,21 @@ __host__ __device__ inline bool row_dp_exact(int gap_open, int gap_ext, int cuto
          gap_open + gap_ext <= kRowMaxScore;
 }
 
+// Whether they are also the faster form.  A row costs one group of four
+// columns at least, so where no gap fits into the X-drop and the band is one
+// column wide, one column at a time is; and a row's share of gap_ext uses up
+// the halves' range, past which an extension starts anew on a warp (after some
+// 1,000 rows of a homolog at kRowMaxGapExt).  One column at a time and grouped,
+// in us: 600,000 extensions with penalties 11/1, X-drop 11 479 and 541, X-drop
+// 12 659 and 577; 300,000 with 11/24, X-drop 38 665 and 615, 120 1,547 and
+// 1,369, 240 3,442 and 3,137; with 11/28, X-drop 60 707 and 683, 120 1,427 and
+// 1,817, 240 2,723 and 2,828; 100,000 with 11/100, X-drop 38 309 and 544.
+constexpr int kRowMaxGapExt = 24;
+
+__host__ __device__ inline bool row_dp_pays(int gap_open, int gap_ext, int cutoff) {
+  return gap_open + gap_ext <= cutoff && gap_ext <= kRowMaxGapExt;
+}
+
 // Whether a matrix entry keeps a pruned cell's diagonal below every
 // threshold and the values of a row inside int16.
 __host__ __device__ __forceinline__ bool row_entry_fits(int v, int gap_ext, int cutoff) {
