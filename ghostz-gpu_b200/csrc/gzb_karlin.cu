@@ -232,14 +232,33 @@ __host__ __device__ constexpr int karlin_steps(int range) {  // scores, a multip
   return (range + kOut) / kOut * kOut;
 }
 
-__global__ void __launch_bounds__(32)
+// The compositions are counted by all warps of the block, 16 bytes a lane,
+// over its queries' residues back to back; one of them goes on alone, on
+// another of the SM's four schedulers in each of the blocks that share it (the
+// first warp of every block: 3,072 queries 160 us, this way 117).  With the
+// block's only warp taking the queries one after the other, a byte a lane,
+// long ones waited: 3,072 queries of 308, 2,000 and 10,000 residues, and of 308
+// with one of 35,000 among them, 117, 147, 279 and 191 us; this way 118, 121,
+// 142 and 119 (a warp a query 156, 155, 160 and 154).
+constexpr int kCountMost = 8;  // warps
+
+// Warps a block, by the blocks an SM gets: as many as fit its registers, and
+// one where the blocks are warps enough (6,144 queries of 308 and of 10,000
+// residues with four warps 138 and 176 us, with one 118 and 225, a warp a query
+// 218 and 228).
+inline int karlin_warps(uint32_t blocks_per_sm) {
+  return blocks_per_sm <= 2 ? kCountMost : blocks_per_sm <= 5 ? 4 : 1;
+}
+
+__global__ void __launch_bounds__(32 * kCountMost, 3)
     karlin_group_kernel(KarlinArgs a, const uint8_t *__restrict__ codes,
                         const uint64_t *__restrict__ offsets,
-                        const uint32_t *__restrict__ lengths, uint32_t n, int rounds,
+                        const uint32_t *__restrict__ lengths, uint32_t n, int rounds, int sms,
                         int32_t *__restrict__ cutoffs, int32_t *__restrict__ triggers,
                         float *__restrict__ karlin) {
   extern __shared__ double columns[];
-  const int lane = threadIdx.x, column = lane % kRow, part = lane / kRow;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+  const int column = lane % kRow, part = lane / kRow;
   const int low = a.low, high = a.high, range = high - low;
   const int steps = karlin_steps(range);
   double *p = columns + column;          // [steps]: zero past the range
@@ -247,23 +266,46 @@ __global__ void __launch_bounds__(32)
   const int rows = rounds * range + 1 + kOut * kGroup;
   const uint32_t r0 = blockIdx.x * kRow, r = r0 + column;
   const int nl = a.number_letters;
-  // compositions (the warp counts one query after the other), then
-  // frequencies with a pseudo-count for absent letters, normalised
+  // compositions, then frequencies with a pseudo-count for absent letters,
+  // normalised
   int *count = reinterpret_cast<int *>(columns + kRow * (2 * steps + kMaxLetters));
-  for (int i = lane; i < 33 * kRow; i += 32) count[i] = 0;
-  const uint64_t offset = r < n ? offsets[r] : 0;
-  const uint32_t length = r < n ? lengths[r] : 0;
-  __syncwarp();
-  for (int k = 0; k < kRow && r0 + k < n; ++k) {
-    const uint8_t *q = codes + __shfl_sync(0xffffffffu, offset, k);
-    const uint32_t len = __shfl_sync(0xffffffffu, length, k);
-#pragma unroll 4
-    for (uint32_t i = lane; i < len; i += 32) {
-      const uint8_t c = q[i];
-      if (c <= kMaxRegular) atomicAdd(&count[33 * k + c], 1);
+  for (int i = threadIdx.x; i < 33 * kRow; i += blockDim.x) count[i] = 0;
+  const uint64_t begin = r < n ? (uint64_t)(codes + offsets[r]) : 0;
+  const uint64_t end = r < n ? begin + lengths[r] : 0;
+  const uint32_t pieces = end > begin ? (uint32_t)((end - (begin & ~15ull) + 15) / 16) : 0;
+  uint32_t last = pieces;  // the pieces of the queries up to the column's
+  for (int d = 1; d < kRow; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, last, d, kRow);
+    if (column >= d) last += t;
+  }
+  const uint32_t all = __shfl_sync(0xffffffffu, last, kRow - 1);
+  __shared__ uint32_t one;
+  if (threadIdx.x == 0) one = 0;
+  __syncthreads();
+  uint32_t slot;  // (its low two bits: the scheduler)
+  asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
+  if (lane == 0 && (slot & 3) == blockIdx.x / sms % 4) one = warp;
+  for (uint32_t i0 = 32 * warp; i0 < all; i0 += blockDim.x) {
+    const uint32_t i = i0 + lane;
+    int k = 0;  // the query piece i is of
+#pragma unroll
+    for (int j = 0; j < kRow - 1; ++j) k += i >= __shfl_sync(0xffffffffu, last, j);
+    const uint32_t first = __shfl_sync(0xffffffffu, last - pieces, k);
+    const uint64_t from = __shfl_sync(0xffffffffu, begin, k), to = __shfl_sync(0xffffffffu, end, k);
+    if (i < all) {
+      // (an aligned piece with a residue of the query in it)
+      const uint64_t at = (from & ~15ull) + 16ull * (i - first);
+      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(at));
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const uint32_t c = (w[j / 4] >> (8 * (j & 3))) & 0xffu;
+        if (c <= kMaxRegular && at + j >= from && at + j < to) atomicAdd(&count[33 * k + c], 1);
+      }
     }
   }
-  __syncwarp();
+  __syncthreads();
+  if (warp != one) return;
   double total = 0.0;
   for (int c = 0; c < nl; ++c) {
     const int k = count[33 * column + c];
@@ -375,9 +417,9 @@ int karlin_rounds(int range, size_t *bytes) {
   return rounds;
 }
 
-// From this many queries on, karlin_group_kernel is the faster: 103 us from 1
-// to 3,000 queries of 308 residues and 133 us of 2,000, where a warp a query
-// takes 94 and 96 at 1,500, 109 and 111 at 2,000, 144 and 147 at 3,000.
+// From this many queries on, karlin_group_kernel is the faster whatever their
+// lengths: 2,048 queries of 50, 308, 2,000 and 10,000 residues 102, 102, 104
+// and 113 us, a warp a query 124, 124, 125 and 129 (1,536 of 308: 107).
 constexpr uint32_t kGroupQueries = 2048;
 // And where its buffers hold the rounds that most queries need (a range of up
 // to 15 scores; a wider one takes a warp a query).
@@ -592,10 +634,11 @@ extern "C" int gzb_query_karlin_cutoffs(const uint8_t *d_codes, const uint64_t *
   if (number_queries >= kGroupQueries && rounds >= kGroupRounds) {
     GZB_CUDA(cudaFuncSetAttribute(karlin_group_kernel,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_group));
-    karlin_group_kernel<<<(number_queries + kRow - 1) / kRow, 32, smem_group,
+    const uint32_t blocks = (number_queries + kRow - 1) / kRow;
+    karlin_group_kernel<<<blocks, 32 * karlin_warps((blocks + sms - 1) / sms), smem_group,
                           (cudaStream_t)stream>>>(
-        a, d_codes, d_offsets, d_lengths, number_queries, rounds, d_cutoffs, d_triggers,
-        d_karlin);
+        a, d_codes, d_offsets, d_lengths, number_queries, rounds, sms, d_cutoffs,
+        d_triggers, d_karlin);
   } else {
     const uint64_t want_fast = (number_queries + kFastWarps - 1) / kFastWarps;
     const uint64_t most_fast = (uint64_t)sms * 8;
