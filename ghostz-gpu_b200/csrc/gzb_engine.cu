@@ -775,6 +775,11 @@ __device__ __forceinline__ void emit_hit(const SeedArgs &a, uint32_t qid, uint32
 constexpr int kSeedBlock = 256;
 constexpr int kUnitsPerWarp = 256;
 
+// The X-drop up to which windows pay.  Seed and member kernels of 1,000 queries
+// x 300,000 proteins, a walk a lane and by windows: X-drop 16 2.33 and 1.94 ms,
+// 25 2.95 and 2.65, 32 3.38 and 3.42, 60 4.84 and 5.61, 127 7.29 and 8.95.
+constexpr int kWindowCutoff = 30;
+
 // Shared memory of a seed-search block: the window and walk tables and the
 // warps' stacks.
 struct SeedShared {
@@ -808,7 +813,6 @@ struct SeedWalker {
   const SeedArgs &a;
   uint32_t window;   // table addresses
   const char *walk;
-  bool fits;         // the matrix (window tables hold entries up to 127)
   WarpStack<uint4> found;     // (database position, entry, its position, cutoff and trigger)
   WarpStack<uint4> open;      // (database position, entry, the window's sides)
   WarpStack<uint2> whole;     // (database position, entry) of whole walks
@@ -821,7 +825,7 @@ struct SeedWalker {
     load_walk_table(sh.walk, a.matrix32, a.p.delimiter);
     window = (uint32_t)__cvta_generic_to_shared(sh.window);
     walk = reinterpret_cast<const char *>(sh.walk);
-    fits = load_window_table(window, a.matrix32, a.p.delimiter);
+    load_window_table(window, a.matrix32, a.p.delimiter);  // (admitted: seed_windows)
     found.item = sh.found[threadIdx.x >> 5];
     open.item = sh.open[threadIdx.x >> 5];
     whole.item = sh.whole[threadIdx.x >> 5];
@@ -850,7 +854,7 @@ struct SeedWalker {
     if (have) {
       ++n_seed;
       const int cutoff = (int)(v.w >> 16), trigger = (int)(int16_t)(v.w & 0xffffu);
-      if (fits && cutoff <= kWalkMaxCutoff) {
+      if (cutoff <= kWalkMaxCutoff) {
         const uint8_t *qs = a.q + v.z, *ds = a.db + v.x;
         uint32_t q[16], d[16];
         WindowWords qw, dw;
@@ -874,9 +878,8 @@ struct SeedWalker {
     if (have) {
       const uint32_t ct = a.L.entry_ct[v.y], side[2] = {v.z, v.w};
       int steps = 0;
-      settled = walk_on(a.q + a.L.entry_cpos[v.y], a.db + v.x, walk,
-                                       (int)(ct >> 16), (int)(int16_t)(ct & 0xffffu), side,
-                                       &steps);
+      settled = walk_on(a.q + a.L.entry_cpos[v.y], a.db + v.x, walk, (int)(ct >> 16),
+                        (int)(int16_t)(ct & 0xffffu), side, &steps);
       if (settled) n_steps += (uint32_t)steps;
     }
     whole.push(have && !settled, make_uint2(v.x, v.y));
@@ -1068,10 +1071,163 @@ member_kernel(SeedArgs a, const uint2 *__restrict__ mwork, uint64_t n_work,
   add_counter(&a.ctr[2], walker.n_steps);
 }
 
+// seed_kernel and member_kernel for wide X-drops (seed_windows): every seed's
+// walk pair by pair on the lane that finds it.  Six blocks per SM (40
+// registers, a few spilled): the loads of long walks want the warps more than
+// the registers.
+__global__ void __launch_bounds__(kSeedBlock, 6)
+seed_lane_kernel(SeedArgs a) {
+  __shared__ __align__(16) int32_t tbl32[kWalkTableBytes / 4];
+  load_walk_table(tbl32, a.matrix32, a.p.delimiter);
+  __syncthreads();
+  const char *tbl = reinterpret_cast<const char *>(tbl32);
+  const int lane = threadIdx.x & 31;
+  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint64_t U = a.units_dev ? *a.units_dev : a.L.n_units;
+  const int thr = a.p.distance_threshold;
+  const int maxmd = a.p.max_member_distance;
+  // a thread's counts stay far below 2^32 (that many walk steps would take
+  // one thread seconds); 32-bit counters leave the six-block register
+  // budget to the walk
+  uint32_t n_dist = 0, n_seed = 0, n_steps = 0;
+  for (uint64_t base = warp * kUnitsPerWarp; base < U; base += nwarps * kUnitsPerWarp) {
+    const uint64_t last = min(base + kUnitsPerWarp, U) - 1;
+    // list range of this warp's units
+    uint64_t l_lo = 0, l_hi = 0;
+    if (lane == 0) {
+      l_lo = upper_segment(a.L.unit_offsets, 0, a.L.n_lists - 1, base);
+      l_hi = upper_segment(a.L.unit_offsets, l_lo, a.L.n_lists - 1, last);
+    }
+    l_lo = __shfl_sync(0xffffffffu, l_lo, 0);
+    l_hi = __shfl_sync(0xffffffffu, l_hi, 0);
+    for (uint64_t u = base + lane; u <= last; u += 32) {
+      const uint64_t l = upper_segment(a.L.unit_offsets, l_lo, l_hi, u);
+      const uint32_t j = (uint32_t)(u - a.L.unit_offsets[l]);
+      const uint32_t pb = a.L.offsets[l], pe = a.L.offsets[l + 1];
+      const uint32_t nchk = a.L.nchk[l];
+      const uint32_t nrep = a.L.rep_count[l];
+      if (j < nrep) {
+        // representative: distance filter for check positions
+        const uint32_t r = a.L.rep_begin[l] + j;
+        const uint32_t rpos = a.X.rep_positions[r];
+        const uint32_t cid = a.X.rep_cluster_ids[r];
+        const bool members = a.X.member_offsets[cid + 1] > a.X.member_offsets[cid];
+        const uint64_t rwin = a.X.rep_windows[r];
+        const uint8_t *dptr = a.db + rpos;
+        for (uint32_t k = pb; k < pe; ++k) {
+          const uint32_t cpos = a.L.entry_cpos[k];
+          const uint8_t *qptr = a.q + cpos;
+          bool try_rep, pass;
+          if (k < pb + nchk) {
+            const int dist = nibble_mismatches(a.L.entry_window[k], rwin);
+            ++n_dist;
+            try_rep = dist <= thr;
+            pass = max(dist - maxmd, 0) <= thr;
+          } else {
+            try_rep = true;
+            pass = true;
+          }
+          if (try_rep) {
+            int steps = 0;
+            ++n_seed;
+            const uint32_t ct = a.L.entry_ct[k];
+            if (walk_hit(qptr, dptr, tbl, (int)(ct >> 16), (int)(int16_t)(ct & 0xffffu),
+                         &steps)) {
+              const uint32_t qid = a.L.entry_qid[k];  // only a hit needs its query
+              emit_hit(a, qid, rpos, cpos - a.q_offsets[qid]);
+            }
+            n_steps += steps;
+          }
+          if (pass && members) append(a.mwork, a.mwork_count, a.mwork_cap, make_uint2(cid, k));
+        }
+      } else {
+        const uint32_t d = a.X.nc_values[a.L.nc_begin[l] + (j - nrep)];
+        const uint8_t *dptr = a.db + d;
+        for (uint32_t k = pb; k < pe; ++k) {
+          const uint32_t cpos = a.L.entry_cpos[k];
+          int steps = 0;
+          ++n_seed;
+          const uint32_t ct = a.L.entry_ct[k];
+          if (walk_hit(a.q + cpos, dptr, tbl, (int)(ct >> 16), (int)(int16_t)(ct & 0xffffu),
+                       &steps)) {
+            const uint32_t qid = a.L.entry_qid[k];  // only a hit needs its query
+            emit_hit(a, qid, d, cpos - a.q_offsets[qid]);
+          }
+          n_steps += steps;
+        }
+      }
+    }
+  }
+  __syncwarp();
+  add_counter(&a.ctr[0], n_dist);
+  add_counter(&a.ctr[1], n_seed);
+  add_counter(&a.ctr[2], n_steps);
+}
+
+__global__ void __launch_bounds__(kSeedBlock, 6)
+member_lane_kernel(SeedArgs a, const uint2 *__restrict__ mwork, uint64_t n_work,
+              const uint64_t *n_dev) {
+  __shared__ __align__(16) int32_t tbl32[kWalkTableBytes / 4];
+  if (n_dev) n_work = *n_dev;
+  load_walk_table(tbl32, a.matrix32, a.p.delimiter);
+  __syncthreads();
+  const char *tbl = reinterpret_cast<const char *>(tbl32);
+  const int lane = threadIdx.x & 31;
+  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  uint32_t n_seed = 0, n_steps = 0;  // per thread, as in seed_lane_kernel
+  for (uint64_t i0 = warp * 32; i0 < n_work; i0 += nwarps * 32) {
+    const uint64_t i = i0 + lane;
+    uint32_t mb = 0, cnt = 0, qid = 0, cpos = 0, ct = 0;
+    if (i < n_work) {
+      const uint2 mw = mwork[i];
+      mb = a.X.member_offsets[mw.x];
+      cnt = a.X.member_offsets[mw.x + 1] - mb;
+      qid = a.L.entry_qid[mw.y];
+      cpos = a.L.entry_cpos[mw.y];
+      ct = a.L.entry_ct[mw.y];
+    }
+    uint32_t incl = cnt;  // inclusive scan of member counts
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += t;
+    }
+    const uint32_t excl = incl - cnt;
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    for (uint32_t base = 0; base < total; base += 32) {
+      const uint32_t p = base + lane;
+      // owner: the last lane whose exclusive offset is <= p (it has p < its
+      // inclusive offset, since every later lane starts beyond p)
+      int o = 0;
+      for (int step = 16; step >= 1; step >>= 1) {
+        const uint32_t e = __shfl_sync(0xffffffffu, excl, o + step);
+        if (o + step < 32 && e <= p) o += step;
+      }
+      const uint32_t m = __shfl_sync(0xffffffffu, mb, o) + (p - __shfl_sync(0xffffffffu, excl, o));
+      const uint32_t sq = __shfl_sync(0xffffffffu, qid, o);
+      const uint32_t sc = __shfl_sync(0xffffffffu, cpos, o);
+      const uint32_t sct = __shfl_sync(0xffffffffu, ct, o);
+      if (p < total) {
+        const uint32_t d = a.X.member_positions[m];
+        int steps = 0;
+        ++n_seed;
+        if (walk_hit(a.q + sc, a.db + d, tbl, (int)(sct >> 16), (int)(int16_t)(sct & 0xffffu),
+                     &steps))
+          emit_hit(a, sq, d, sc - a.q_offsets[sq]);
+        n_steps += steps;
+      }
+    }
+  }
+  __syncwarp();
+  add_counter(&a.ctr[1], n_seed);
+  add_counter(&a.ctr[2], n_steps);
+}
+
 // ---------------------------------------------------------------------------
-// Dealt seed walker.  seed_kernel gives each lane whole units (a unit's
-// every list entry in turn), so a warp waits for its lane with the longest
-// list.  Here the seeds of 32 units -- every (unit, list entry) pair -- form
+// Dealt seed walker.  seed_lane_kernel gives each lane whole units (a unit's
+// every list entry in turn) and walks a seed where it finds it, so a warp waits
+// for its lane with the longest list.  Here the seeds of 32 units -- every (unit, list entry) pair -- form
 // one stream that is dealt to the lanes 32 at a time, as member_kernel deals
 // member seeds: a warp then waits only for the longest single walk of a
 // round.  A lane finds its seed's unit with a shuffle search over the
@@ -1875,6 +2031,7 @@ struct gzb_engine {
   DevParams dp{};
   bool have_params = false;
   DBuf matrix32;
+  bool window_matrix = false;  // its entries fit the window tables
   // database
   int32_t chunk_id = 0;
   DBuf db_buf;
@@ -1888,6 +2045,7 @@ struct gzb_engine {
   DBuf q_buf, q_offsets, q_lengths, q_cut, q_trig;
   DBuf q_off64, q_prep;  // query preparation on the device: 64-bit offsets, scratch
   DBuf q_prev, q_next;  // nearest delimiters of every query position
+  uint32_t wide_queries = 0;  // with an X-drop above kWindowCutoff
   uint64_t q_len = 0;
   uint32_t nq = 0;
   uint32_t max_qlen = 0;
@@ -2041,11 +2199,15 @@ __global__ void code_range_kernel(const uint8_t *p, uint64_t n, unsigned int *ba
   if (acc & 0xE0E0E0E0u) atomicOr(bad, 1u);
 }
 
-// the query cutoffs the engine takes (1..32767) and triggers (int16)
+// the query cutoffs the engine takes (1..32767) and triggers (int16): sets
+// flags[0] for others, and counts the cutoffs above kWindowCutoff in flags[1]
 __global__ void cutoff_range_kernel(const int32_t *cut, const int32_t *trig, uint32_t n,
-                                    unsigned int *bad) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    if (cut[i] < 1 || cut[i] > 32767 || trig[i] < -32768 || trig[i] > 32767) atomicOr(bad, 1u);
+                                    unsigned int *flags) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    if (cut[i] < 1 || cut[i] > 32767 || trig[i] < -32768 || trig[i] > 32767)
+      atomicOr(flags, 1u);
+    if (cut[i] > kWindowCutoff) atomicAdd(flags + 1, 1u);
+  }
 }
 
 // cut[idx[i]] = c[i], trig[idx[i]] = t[i]
@@ -2245,6 +2407,8 @@ extern "C" int gzb_engine_set_params(gzb_engine *e, const gzb_params *p) {
       m[r * 32 + c] = p->score_matrix[r * p->number_letters + c];
   GZB_TRY(e->matrix32.ensure(sizeof(m)));
   GZB_CUDA(cudaMemcpy(e->matrix32.p, m, sizeof(m), cudaMemcpyHostToDevice));
+  e->window_matrix = true;
+  for (int32_t v : m) e->window_matrix = e->window_matrix && abs(v) <= kWalkMaxEntry;
   e->have_params = true;
   return GZB_OK;
 }
@@ -2810,7 +2974,7 @@ gzb_engine *e, const uint8_t *codes, uint64_t length,
   GZB_CHECK(length < (1ull << 31), GZB_ERR_OVERFLOW, "query buffer exceeds 2^31 residues");
   cudaStream_t s = (cudaStream_t)stream;
   e->have_queries = false;
-  uint32_t maxl = 0;
+  uint32_t maxl = 0, wide = 0;
   for (uint32_t i = 0; i < number_queries; ++i) {
     GZB_CHECK(lengths[i] >= 2 && (uint64_t)offsets[i] + lengths[i] <= length, GZB_ERR_INVALID,
               "query %u outside the buffer", i);
@@ -2824,7 +2988,9 @@ gzb_engine *e, const uint8_t *codes, uint64_t length,
     GZB_CHECK(triggers[i] >= -32768 && triggers[i] <= 32767, GZB_ERR_INVALID,
               "gapped trigger of query %u outside int16", i);
     maxl = std::max(maxl, lengths[i]);
+    wide += cutoffs[i] > kWindowCutoff;
   }
+  e->wide_queries = wide;
   e->nq = number_queries;
   e->q_len = length;
   e->max_qlen = maxl;
@@ -2886,7 +3052,7 @@ extern "C" int gzb_engine_set_protein_queries(gzb_engine *e, const uint8_t *code
   GZB_TRY(e->q_cut.ensure(4 * (uint64_t)number_queries));
   GZB_TRY(e->q_trig.ensure(4 * (uint64_t)number_queries));
   uint8_t *q = e->q_buf.as<uint8_t>() + kPad;
-  unsigned int *flags = e->codeflag.as<unsigned int>();  // codes, SEG status, cutoffs
+  unsigned int *flags = e->codeflag.as<unsigned int>();  // codes, SEG status, cutoffs, wide ones
   if (filter)
     GZB_TRY(gzb_seg_protein_queries(q, e->q_off64.as<uint64_t>(), e->q_lengths.as<uint32_t>(),
                                     number_queries, flags + 1, s));
@@ -2941,13 +3107,14 @@ extern "C" int gzb_engine_set_protein_queries(gzb_engine *e, const uint8_t *code
   if (triggers)
     GZB_CUDA(cudaMemcpyAsync(triggers, e->q_trig.p, 4 * (uint64_t)number_queries,
                              cudaMemcpyDeviceToHost, s));
-  unsigned int bad[3] = {0, 0, 0};
-  GZB_CUDA(cudaMemcpyAsync(bad, flags, 12, cudaMemcpyDeviceToHost, s));
+  unsigned int bad[4] = {0, 0, 0, 0};
+  GZB_CUDA(cudaMemcpyAsync(bad, flags, 16, cudaMemcpyDeviceToHost, s));
   GZB_CUDA(cudaStreamSynchronize(s));
   GZB_CHECK(bad[0] == 0, GZB_ERR_INVALID, "residue codes must be below 32 (after SEG)");
   GZB_CHECK(bad[1] == 0, GZB_ERR_INVALID, "SEG left %u queries unmasked", bad[1]);
   GZB_CHECK(bad[2] == 0, GZB_ERR_INVALID,
             "a query's cutoff is outside 1..32767 or its trigger outside int16");
+  e->wide_queries = bad[3];
   return build_query_lists(e, length, number_queries, s);
 }
 
@@ -3007,7 +3174,7 @@ extern "C" int gzb_engine_set_translated_queries(gzb_engine *e, const uint8_t *d
   GZB_TRY(e->q_trig.ensure(4 * (uint64_t)n));
   uint8_t *q = e->q_buf.as<uint8_t>() + kPad;
   const uint32_t *d_read_len = reinterpret_cast<const uint32_t *>(base + at_len);
-  unsigned int *flags = e->codeflag.as<unsigned int>();  // codes, SEG status, cutoffs
+  unsigned int *flags = e->codeflag.as<unsigned int>();  // codes, SEG status, cutoffs, wide ones
   GZB_TRY(gzb_translate_dna_queries(base, reinterpret_cast<const uint64_t *>(base + at_off),
                                     d_read_len, n, e->q_off64.as<uint64_t>(), delim, q, s));
   if (filter)
@@ -3026,13 +3193,14 @@ extern "C" int gzb_engine_set_translated_queries(gzb_engine *e, const uint8_t *d
     GZB_CUDA(cudaMemcpyAsync(cutoffs, e->q_cut.p, 4ull * n, cudaMemcpyDeviceToHost, s));
   if (triggers)
     GZB_CUDA(cudaMemcpyAsync(triggers, e->q_trig.p, 4ull * n, cudaMemcpyDeviceToHost, s));
-  unsigned int bad[3] = {0, 0, 0};
-  GZB_CUDA(cudaMemcpyAsync(bad, flags, 12, cudaMemcpyDeviceToHost, s));
+  unsigned int bad[4] = {0, 0, 0, 0};
+  GZB_CUDA(cudaMemcpyAsync(bad, flags, 16, cudaMemcpyDeviceToHost, s));
   GZB_CUDA(cudaStreamSynchronize(s));
   GZB_CHECK(bad[0] == 0, GZB_ERR_INVALID, "residue codes must be below 32");
   GZB_CHECK(bad[1] == 0, GZB_ERR_INVALID, "SEG left %u frames unmasked", bad[1]);
   GZB_CHECK(bad[2] == 0, GZB_ERR_INVALID,
             "a query's cutoff is outside 1..32767 or its trigger outside int16");
+  e->wide_queries = bad[3];
   return build_query_lists(e, total, n, s);
 }
 
@@ -3058,6 +3226,18 @@ int launch_chain(gzb_engine *e, uint32_t nq, uint64_t *hits, const uint64_t *beg
       smem_slots);
   GZB_CUDA(cudaGetLastError());
   return GZB_OK;
+}
+
+// Whether the seed kernels evaluate windows: the tables hold the matrix, and
+// most queries' walks mostly end inside a window (kWindowCutoff).
+bool seed_windows(const gzb_engine *e) {
+  return e->window_matrix && 2ull * e->wide_queries <= e->nq;
+}
+auto seed_kernel_of(const gzb_engine *e) {
+  return seed_windows(e) ? seed_kernel : seed_lane_kernel;
+}
+auto member_kernel_of(const gzb_engine *e) {
+  return seed_windows(e) ? member_kernel : member_lane_kernel;
 }
 
 int presearch_impl(gzb_engine *e, int schedule, cudaStream_t s) {
@@ -3125,7 +3305,7 @@ int presearch_impl(gzb_engine *e, int schedule, cudaStream_t s) {
       if (stile.seed_walker == GZB_SEED_WALKER_DEALT)
         seed_dealt_kernel<<<grid1(warps * 32, kSeedBlock, 148 * 16), kSeedBlock, 0, s>>>(a);
       else
-        seed_kernel<<<grid1(warps * 32, kSeedBlock, 148 * 16), kSeedBlock, 0, s>>>(a);
+        seed_kernel_of(e)<<<grid1(warps * 32, kSeedBlock, 148 * 16), kSeedBlock, 0, s>>>(a);
       GZB_CUDA(cudaGetLastError());
       ++launches;
     }
@@ -3146,8 +3326,8 @@ int presearch_impl(gzb_engine *e, int schedule, cudaStream_t s) {
                             e->mwork_alt.as<uint64_t>(), n_mwork, bits_for(X.n_reps + 1), s,
                             &sorted_mw));
       launches += 1;
-      member_kernel<<<grid1((n_mwork + 31) / 32 * 32, kSeedBlock, 148 * 16), kSeedBlock, 0,
-                      s>>>(a, reinterpret_cast<const uint2 *>(sorted_mw), n_mwork, nullptr);
+      member_kernel_of(e)<<<grid1((n_mwork + 31) / 32 * 32, kSeedBlock, 148 * 16), kSeedBlock, 0,
+                            s>>>(a, reinterpret_cast<const uint2 *>(sorted_mw), n_mwork, nullptr);
       GZB_CUDA(cudaGetLastError());
       ++launches;
       GZB_CUDA(cudaMemcpyAsync(hctr, c, 64, cudaMemcpyDeviceToHost, s));
@@ -3536,7 +3716,7 @@ int graph_body(gzb_engine *e, int schedule, const GappedTile &tile, bool learned
     if (tile.seed_walker == GZB_SEED_WALKER_DEALT)
       seed_dealt_kernel<<<148 * 16, kSeedBlock, 0, s>>>(a);
     else
-      seed_kernel<<<148 * 16, kSeedBlock, 0, s>>>(a);
+      seed_kernel_of(e)<<<148 * 16, kSeedBlock, 0, s>>>(a);
     GZB_CUDA(cudaGetLastError());
     ++launches;
   }
@@ -3550,7 +3730,7 @@ int graph_body(gzb_engine *e, int schedule, const GappedTile &tile, bool learned
   GZB_TRY(sort_keys_u64(e, reinterpret_cast<uint64_t *>(a.mwork), e->mwork_alt.as<uint64_t>(),
                         c.mwork, bits_for(X.n_reps + 1), s, &sorted_mw));
   ++launches;
-  member_kernel<<<148 * 16, kSeedBlock, 0, s>>>(
+  member_kernel_of(e)<<<148 * 16, kSeedBlock, 0, s>>>(
       a, reinterpret_cast<const uint2 *>(sorted_mw), c.mwork, plan + 0);
   GZB_CUDA(cudaGetLastError());
   ++launches;
@@ -3685,7 +3865,7 @@ uint64_t graph_key(const gzb_engine *e, int schedule, const GappedTile &tile, bo
                         (uint64_t)(uintptr_t)e->spill, e->spill_cap,
                         (uint64_t)(uintptr_t)e->band_pool, (uint64_t)(uintptr_t)e->gcounters,
                         (uint64_t)(uintptr_t)e->gcells, (uint64_t)(uintptr_t)e->report_h,
-                        (uint64_t)learned};
+                        (uint64_t)learned, (uint64_t)seed_windows(e)};
   return fnv_mix(h, v, sizeof(v));
 }
 
