@@ -196,14 +196,14 @@ __device__ void tb_extend(const TbArgs &a, const int *sm, const TbSide &t, int2 
 }
 
 constexpr int kTbWarpColumns = 256;  // circular band of one warp (int2 columns)
-constexpr int kTbMaxBand = kTbWarpColumns - 32;  // (residues are read 32 columns ahead)
+constexpr int kTbWarpResidues = 512;  // its residues (read 32 columns ahead)
 constexpr int kTbWarpsPerBlock = 8;
 static_assert(kTbWarpBlock == kTbWarpsPerBlock * 32, "launch block of the warp kernels");
 
 // A warp's band: the cells and the query residues of its columns.
 struct TbBand {
   int2 cell[kTbWarpColumns];
-  uint8_t res[kTbWarpColumns];
+  uint8_t res[kTbWarpResidues];
 };
 
 // tb_extend by one warp (lanes must all call it with the same side); it
@@ -211,8 +211,8 @@ struct TbBand {
 // ops_cap bytes and rows_cap rows that need not be zeroed: every byte of a
 // row's range is written (0 for a pruned cell and the sentinel, as a fresh
 // GappedExtender holds), and the bytes past the last row up to *ops_bytes
-// are zeroed at the end.  Returns false when the band outgrows kTbMaxBand or
-// the side outgrows the storage (outputs then meaningless).
+// are zeroed at the end.  Returns false when the band outgrows kTbWarpColumns
+// or the side outgrows the storage (outputs then meaningless).
 //
 // A row's latency is what long sides wait for and its instructions are what
 // many short ones cost, so a chunk of 32 columns runs only the scans that can
@@ -240,8 +240,8 @@ __device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, 
                                uint8_t *ops, uint32_t *row_meta, uint64_t ops_cap,
                                uint32_t rows_cap, uint64_t *ops_bytes, uint32_t *rows,
                                int *best_score, int *best_p0, int *best_p1) {
-  constexpr int W = kTbMaxBand;
-  constexpr int wmask = kTbWarpColumns - 1;
+  constexpr int W = kTbWarpColumns;
+  constexpr int wmask = W - 1, rmask = kTbWarpResidues - 1;
   constexpr unsigned full = 0xffffffffu;
   constexpr int kFar = 1 << 30;
   const int lane = threadIdx.x & 31;
@@ -266,7 +266,7 @@ __device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, 
     while (seen < c && delim_at == kFar) {
       const int k = seen + 1 + lane;
       const int r = q0[(k - 1) * inc];
-      band.res[k & wmask] = (uint8_t)r;
+      band.res[k & rmask] = (uint8_t)r;
       const unsigned m = __ballot_sync(full, r == delim);
       if (m) delim_at = seen + __ffs(m);
       seen += 32;
@@ -330,7 +330,7 @@ __device__ bool tb_extend_warp(const TbArgs &a, const int *sm, const TbSide &t, 
       int qres = 0;
       if (active) {
         st = band.cell[c & wmask];
-        qres = band.res[c & wmask];
+        qres = band.res[c & rmask];
       }
       int prev = __shfl_up_sync(full, st.x, 1);
       if (lane == 0) prev = diag;
@@ -597,7 +597,7 @@ __global__ void tb_order_kernel(uint64_t n_sides, const uint32_t *bucket_sides,
 // sides gather; then each lane walks one of them (PickOptimalPath and
 // BuildResult's counts), the 32 walks in parallel, and the scratch is
 // reused.  A side the warp cannot run exactly (X-drop >= 1024, a band wider
-// than kTbMaxBand) or whose storage outgrows an empty scratch is
+// than kTbWarpColumns) or whose storage outgrows an empty scratch is
 // flagged in `redo` with its sizes left to the thread kernels; the others
 // get zero sizes.  `order` (or null: side after side): the sides to run, the
 // next of them to whichever warp is free.
