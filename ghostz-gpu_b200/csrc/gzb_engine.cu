@@ -3236,6 +3236,14 @@ int launch_chain(gzb_engine *e, uint32_t nq, uint64_t *hits, const uint64_t *beg
   return GZB_OK;
 }
 
+// Whether the grouped rows of the gapped extension admit the score matrix.
+bool rows_admit(const gzb_params &p) {
+  bool fits = true;
+  for (int i = 0; i < p.number_letters * p.number_letters; ++i)
+    fits = fits && row_entry_fits(p.score_matrix[i], p.gap_extension, p.gapped_cutoff);
+  return fits;
+}
+
 // Whether the seed kernels evaluate windows: the tables hold the matrix, and
 // most queries' walks mostly end inside a window (kWindowCutoff).
 bool seed_windows(const gzb_engine *e) {
@@ -3432,6 +3440,7 @@ int presearch_impl(gzb_engine *e, int schedule, cudaStream_t s) {
     job.gap_open = e->params.gap_open;
     job.gap_ext = e->params.gap_extension;
     job.cutoff = e->params.gapped_cutoff;
+    job.general = !rows_admit(e->params);
     if (want_feat) {
       GZB_TRY(e->efeat.ensure(4 * kFeat * (next + 1)));
       ext_features_kernel<<<grid1(n_surv, 256), 256, 0, s>>>(
@@ -3789,6 +3798,7 @@ int graph_body(gzb_engine *e, int schedule, const GappedTile &tile, bool learned
   job.gap_open = e->params.gap_open;
   job.gap_ext = e->params.gap_extension;
   job.cutoff = e->params.gapped_cutoff;
+  job.general = !rows_admit(e->params);
   GappedTile t = tile;
   if (schedule == GZB_SCHEDULE_PLAIN) t.kernel = GZB_GAPPED_KERNEL_STATIC;
   const uint32_t *order = nullptr;

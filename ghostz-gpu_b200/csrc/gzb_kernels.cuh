@@ -411,6 +411,7 @@ struct GappedJob {
   const uint8_t *query;     // concatenated queries
   const uint8_t *db;        // database chunk
   int delim, gap_open, gap_ext, cutoff;
+  bool general = false;     // the host knows of entries the grouped rows do not admit
 };
 
 // Tile of the presearch: the gapped stage's one-thread-per-extension kernel

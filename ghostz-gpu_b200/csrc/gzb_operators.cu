@@ -311,6 +311,8 @@ struct LaneWork<W, false> {
   __device__ __forceinline__ int step(const GappedJob &job, int st) {
     return st == kLaneRunning ? lane_row(job, tbl, band, x) : st;
   }
+  // whether the lane has to step on (alone)
+  __device__ __forceinline__ bool any(bool running) const { return running; }
   __device__ __forceinline__ bool overflow(int st) const { return st == kLaneOverflow || x.ovf; }
   __device__ __forceinline__ int score() const { return x.maxs; }
   __device__ __forceinline__ int pos0() const { return x.mp0; }
@@ -337,17 +339,32 @@ struct LaneWork<W, true> {
   __device__ __forceinline__ int step(const GappedJob &job, int st) {
     return row_step<W, kLaneBlock>(job, tbl, band, x, st);
   }
+  // whether the lane has to step on (with its warp)
+  __device__ __forceinline__ bool any(bool running) const {
+    return __any_sync(0xffffffffu, running) != 0;
+  }
   __device__ __forceinline__ bool overflow(int st) const { return st == kLaneOverflow; }
   __device__ __forceinline__ int score() const { return x.best; }
   __device__ __forceinline__ int pos0() const { return x.pos0(); }
   __device__ __forceinline__ int pos1() const { return x.pos1(); }
 };
 
+// (out of line in the persistent kernels, whose grouped rows took 2.5 % longer
+// with both forms inlined; the static one's took 1.5 % longer with this)
+template <int W, class Run>
+__device__ __noinline__ void general_lane_work(const GappedJob &job, int *tbl, uint32_t *cells,
+                                               uint8_t *res, const int32_t *matrix,
+                                               int number_letters, int stride, Run run) {
+  LaneWork<W, false> x(job, tbl, cells, res, matrix, number_letters, stride);
+  run(x);
+}
+
 // run(the extension state of this thread).  The matrix may be known to the
 // device alone, so a FAST kernel holds the other form, too: 600,000
-// extensions with -2000 for the stop letter 11.4 ms, handed on to the warp
-// kernel 17.4.
-template <int W, bool FAST, class Run>
+// extensions with -2000 for the stop letter 12.0 ms (11.4 in a kernel of its
+// own, which an engine runs: GappedJob::general), handed on to the warp kernel
+// 17.4.
+template <int W, bool FAST, bool APART = true, class Run>
 __device__ __forceinline__ void with_lane_work(const GappedJob &job, int *tbl, uint32_t *cells,
                                                uint8_t *res, const int32_t *matrix,
                                                int number_letters, int stride, Run run) {
@@ -358,8 +375,12 @@ __device__ __forceinline__ void with_lane_work(const GappedJob &job, int *tbl, u
       return;
     }
   }
-  LaneWork<W, false> x(job, tbl, cells, res, matrix, number_letters, stride);
-  run(x);
+  if constexpr (FAST && APART) {
+    general_lane_work<W>(job, tbl, cells, res, matrix, number_letters, stride, run);
+  } else {
+    LaneWork<W, false> x(job, tbl, cells, res, matrix, number_letters, stride);
+    run(x);
+  }
 }
 
 template <bool FAST>
@@ -373,7 +394,7 @@ gapped_lane_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
   __shared__ __align__(16) uint32_t cells_s[kLaneW * kLaneBlock];
   __shared__ __align__(4) uint8_t res_s[kLaneW * kLaneBlock];
   if (n_dev) n = *n_dev;
-  auto run = [&](auto &x) {
+  auto run = [=](auto &x) {
     unsigned long long cells = 0;
     const size_t lane = threadIdx.x & 31;
     for (size_t i0 = blockIdx.x * (size_t)blockDim.x + (threadIdx.x & ~31u); i0 < n;
@@ -388,7 +409,7 @@ gapped_lane_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
         d = dpos[e];
         st = x.init(job, q, d, rev);
       }
-      while (__any_sync(0xffffffffu, st == kLaneRunning)) st = x.step(job, st);
+      while (x.any(st == kLaneRunning)) st = x.step(job, st);
       if (i >= n) {
       } else if (x.overflow(st)) {
         spill[atomicAdd(spill_count, 1u)] = e;
@@ -408,7 +429,8 @@ gapped_lane_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
     cells += __shfl_down_sync(0xffffffffu, cells, 1);
     if ((threadIdx.x & 31) == 0 && cells) atomicAdd(cells_total, cells);
   };
-  with_lane_work<kLaneW, FAST>(job, sm, cells_s, res_s, matrix, number_letters, stride, run);
+  with_lane_work<kLaneW, FAST, false>(job, sm, cells_s, res_s, matrix, number_letters, stride,
+                                      run);
 }
 
 // Flattened one-thread-per-extension kernel over a device work queue
@@ -450,7 +472,7 @@ gapped_lane_queue_kernel(GappedJob job, const int32_t *__restrict__ matrix, int 
   __shared__ __align__(16) uint32_t cells_s[kLaneW * kLaneBlock];
   __shared__ __align__(4) uint8_t res_s[kLaneW * kLaneBlock];
   if (n_dev) n = *n_dev;
-  auto run = [&](auto &x) {
+  auto run = [=](auto &x) {
     const int lane = threadIdx.x & 31;
     unsigned long long cells = 0;
     for (;;) {
@@ -468,7 +490,7 @@ gapped_lane_queue_kernel(GappedJob job, const int32_t *__restrict__ matrix, int 
         d = dpos[e];
         st = x.init(job, q, d, rev);
       }
-      while (__any_sync(0xffffffffu, st == kLaneRunning)) st = x.step(job, st);
+      while (x.any(st == kLaneRunning)) st = x.step(job, st);
       if (i < n) {
         if (x.overflow(st)) {
           spill[atomicAdd(spill_count, 1u)] = e;
@@ -528,7 +550,7 @@ gapped_rows_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
   uint32_t *cells_s = kStatic ? cells_st : reinterpret_cast<uint32_t *>(rows_band);
   uint8_t *res_s = kStatic ? res_st : rows_band + (size_t)W * kLaneBlock * 4;
   if (n_dev) n = *n_dev;
-  auto run = [&](auto &x) {
+  auto run = [=](auto &x) {
     uint32_t e = 0, q = 0, d = 0;
     bool have = false, done = false;
     unsigned long long cells = 0;
@@ -590,7 +612,7 @@ gapped_deal_kernel(GappedJob job, const int32_t *__restrict__ matrix, int number
   __shared__ __align__(16) uint32_t cells_s[kLaneW * kLaneBlock];
   __shared__ __align__(4) uint8_t res_s[kLaneW * kLaneBlock];
   if (n_dev) n = *n_dev;
-  auto run = [&](auto &x) {
+  auto run = [=](auto &x) {
     const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
     uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     // the next extension of this lane, loaded one extension ahead
@@ -752,7 +774,7 @@ static int launch_gapped_rows_as(const GappedTile &tile, const GappedJob &job,
 }
 
 static bool grouped_rows(const GappedJob &job) {
-  return row_dp_exact(job.gap_open, job.gap_ext, job.cutoff) &&
+  return !job.general && row_dp_exact(job.gap_open, job.gap_ext, job.cutoff) &&
          row_dp_pays(job.gap_open, job.gap_ext, job.cutoff);
 }
 

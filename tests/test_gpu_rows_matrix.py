@@ -6,6 +6,7 @@ import pytest
 
 from gzb import params as P
 from gzb import workload as W
+from kernel_trace import kernels
 from test_gpu_operators import _concat, _gapped_gpu, torch_cuda  # noqa: F401
 
 pytestmark = pytest.mark.gpu
@@ -67,5 +68,8 @@ def test_engine_hands_nothing_on(torch_cuda, kernel):  # noqa: F811
         c = e.counters()
         assert c["gapped_extensions"] > 50
         assert c["gapped_fallbacks"] == 0
+        e.reset_results()
+        names = kernels(lambda: e.presearch(N.SCHEDULE_BATCHED))
+        assert not any("gapped" in n and "true>" in n for n in names)
     finally:
         e.close()
