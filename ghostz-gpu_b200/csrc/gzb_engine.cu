@@ -142,6 +142,7 @@ __device__ __forceinline__ void load_hash_codes(const DevParams &p, int *codes) 
 }
 
 constexpr int kHashResidues = 8;  // hashes of up to this many residues run in registers
+constexpr int kHashMaxScore = (1 << 23) - 1;  // and of code scores that load_hash_codes packs
 
 // seed_hash of the residues whose codes are v[0 ..]; max_hash_length <=
 // kHashResidues
@@ -193,7 +194,7 @@ __device__ __forceinline__ void append_some(uint64_t *buf, unsigned long long *c
 // Keep rule of the index build (:85-108): a k-mer is dropped when the next
 // position's k-mer is contained in it.  A thread takes four positions from
 // three words of the chunk (aligned: the chunk starts on a 256-byte
-// boundary); hashes longer than kHashResidues (REGISTERS false) are read
+// boundary); other hashes (REGISTERS false, see hash_in_registers) are read
 // residue by residue.  One position a thread from byte loads, an atomic for
 // every 32: 6.9 ms for 72 M residues, this 0.54 ms.
 template <bool REGISTERS>
@@ -2284,6 +2285,12 @@ int build_csr(gzb_engine *e, const uint64_t *pairs, uint64_t n, uint32_t **keys,
   return GZB_OK;
 }
 
+bool hash_in_registers(const DevParams &p) {
+  bool fits = p.max_hash_length <= kHashResidues;
+  for (int v : p.code_scores) fits = fits && v >= -kHashMaxScore && v <= kHashMaxScore;
+  return fits;
+}
+
 int check_engine(gzb_engine *e) {
   GZB_CHECK(e, GZB_ERR_INVALID, "null engine");
   GZB_CUDA(cudaSetDevice(e->device));
@@ -2472,8 +2479,7 @@ extern "C" int gzb_engine_set_database(gzb_engine *e, int32_t chunk_id, const ui
   GZB_TRY(pairs_alt.ensure(8 * (length + 1)));
   GZB_TRY(e->ctr.ensure(64));
   GZB_CUDA(cudaMemsetAsync(e->ctr.p, 0, 64, s));
-  auto db_pairs = e->dp.max_hash_length <= kHashResidues ? db_pairs_kernel<true>
-                                                         : db_pairs_kernel<false>;
+  auto db_pairs = hash_in_registers(e->dp) ? db_pairs_kernel<true> : db_pairs_kernel<false>;
   db_pairs<<<grid1((length + 3) / 4, 256, 148 * 64), 256, 0, s>>>(
       e->dp, db, length, pairs.as<uint64_t>(), e->ctr.as<unsigned long long>());
   GZB_CUDA(cudaGetLastError());
@@ -2897,8 +2903,8 @@ int build_query_lists(gzb_engine *e, uint64_t length, uint32_t number_queries, c
   GZB_TRY(alt.ensure(8 * (length + 1)));
   GZB_TRY(e->ctr.ensure(64));
   GZB_CUDA(cudaMemsetAsync(e->ctr.p, 0, 8, s));
-  auto query_entries = e->dp.max_hash_length <= kHashResidues ? query_entries_kernel<true>
-                                                              : query_entries_kernel<false>;
+  auto query_entries = hash_in_registers(e->dp) ? query_entries_kernel<true>
+                                                : query_entries_kernel<false>;
   query_entries<<<grid1((length + 3) / 4, 256), 256, 0, s>>>(
       e->dp, e->q_buf.as<uint8_t>() + kPad, e->q_prev.as<uint32_t>(), e->q_next.as<uint32_t>(),
       length, keys.as<uint64_t>(), e->ctr.as<unsigned long long>(), length + 1);
