@@ -1452,7 +1452,6 @@ chain_kernel(DevParams p, const uint8_t *__restrict__ q, const uint8_t *__restri
 __device__ __forceinline__ uint32_t subject_of(const uint32_t *off, uint32_t nseq,
                                                uint32_t db_len, uint32_t pos);
 
-// Extension list of the chained hits: one warp per query, lanes over its
 // For every position p of a query in the concatenated buffer: the nearest
 // delimiter at or before p (prev) and at or after p (next), within the
 // query (its first and last codes are delimiters).  One warp per query,
@@ -1495,6 +1494,7 @@ __global__ void delim_dist_kernel(const uint8_t *q, const uint32_t *offsets,
   }
 }
 
+// Extension list of the chained hits: one warp per query, lanes over its
 // kept hits (database order).  Reverse extension of hit h at h, forward at
 // n_surv + h; neighbours[h] counts the query's kept hits within 256
 // database residues of h (a cost-model feature).

@@ -104,7 +104,7 @@ __global__ void distance_kernel(const uint8_t *__restrict__ q,
 // half's range are walked pair by pair (kWalkMaxDrop: what a delimiter's
 // entry of the walk table still ends).
 // 3,000,000 seeds of 2,048 queries: 306 us with a walk a thread, this
-// 195 (50,000 seeds: 20.6 and 13.5); of these seeds 85 in 100 are hits, nearly
+// 196 (50,000 seeds: 20.6 and 13.5); of these seeds 85 in 100 are hits, nearly
 // all settled by their windows.
 constexpr int kUngappedBlock = 256;
 constexpr int kWalkMaxDrop = -kWalkDelim;

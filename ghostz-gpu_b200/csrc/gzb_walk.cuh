@@ -221,12 +221,12 @@ __device__ __forceinline__ bool walk_on(const uint8_t *q, const uint8_t *d, cons
   }
   if (side[0] == kSideUnknown || best[0] + best[1] > trigger) return false;
   if (!(side[0] >> 31))
-    best[0] = walk_side<-1>(q - 1 - kWindow, d - 1 - kWindow, tbl, cutoff,
-                               trigger - best[1], &n, best[0] - (int)(side[0] & 0xffffu), best[0]);
+    best[0] = walk_side<-1>(q - 1 - kWindow, d - 1 - kWindow, tbl, cutoff, trigger - best[1], &n,
+                            best[0] - (int)(side[0] & 0xffffu), best[0]);
   if (best[0] + best[1] > trigger) return false;
   if (!(side[1] >> 31))
     best[1] = walk_side<1>(q + kWindow, d + kWindow, tbl, cutoff, trigger - best[0], &n,
-                              best[1] - (int)(side[1] & 0xffffu), best[1]);
+                           best[1] - (int)(side[1] & 0xffffu), best[1]);
   *steps = n;
   return best[0] + best[1] <= trigger;
 }
